@@ -1,0 +1,367 @@
+// BiCGSTAB with the matrix resident on the SMs (the reference's default solver, Simulation.cpp:49-53:
+// Jacobi preconditioner, zero start, tolerance DBL_EPSILON on the recursive residual, at most 2N
+// iterations, shadow-residual restart): the whole solve in one cooperative launch, for systems whose
+// matrix fits the register files and shared memories of the GPU (N <= 2048: 33.6 MB).
+//
+// What bounds it: at these sizes a product reads nothing from outside the SM and takes well under a
+// microsecond, so an iteration costs its two all-to-all exchanges and the chain of dot products.
+//   * A CTA owns 16 rows (or N / SMs, if that is more), a thread up to 28 entries of one row in
+//     registers and the rest in shared memory.  Few CTAs: every CTA reads every published vector, and
+//     with 16 rows the slots of a CTA fill whole 128-byte lines, which are polled by all the others.
+//     Measured at N = 812, per iteration: 6.1 us with 16 rows, 7.0 with 8, 7.8 with 12 and 8.3 with 6
+//     (one CTA per SM).
+//   * Every CTA keeps all of r, p, v (in registers, the same elements in the same thread everywhere) and
+//     updates them redundantly, in the same order, so every CTA holds the same bits and takes the same
+//     decisions.  That leaves two exchanges per iteration (v = A y and t = A z) instead of the five
+//     grid barriers of k_pbicg (bicg.cu).
+//   * An exchange has no barrier: a published element is a 16-byte slot {value, sequence number}, written
+//     and read as one 128-bit access, and a reader polls the slots it needs until they carry the current
+//     number.  Two sets of slots by the number's parity suffice: a CTA publishes number s + 2 only after
+//     it has read all of s + 1, which every other CTA published after it had read all of s.  Sequence
+//     numbers grow over the context's solves, so the slots are cleared only when they are allocated.
+//     1.3 to 1.8 us per exchange over 50 to 140 CTAs; a counter barrier and a read of the vector take
+//     1.9 to 2.4 us.
+// Measured (B200, whole solve, against k_pbicg in batches of 64 iterations): N = 162: 0.10 ms (0.63),
+// N = 812 with the wall image: 0.23 ms (1.13), N = 1442: 0.35 ms (1.66), N = 1962: 0.59 ms.
+//
+// A wait is bounded (Ctx::wait_limit): a warp that gives up sets the error word and its CTA returns; the
+// others then run out of their own waits.  The host finishes the solve with the multi-kernel form.
+#include <math.h>
+
+#include <algorithm>
+
+#include "ctx.h"
+
+namespace bemb {
+
+namespace {
+
+constexpr int RB_T = 512;
+constexpr int RB_WARPS = RB_T / 32;
+constexpr double RB_EPS = 2.220446049250313080847e-16;
+
+struct RBArgs {
+    int n, rows, nv, npart, maxit;  // rows per CTA; doubles of the input vector and of the row partials
+    const double* A;
+    const double* b;
+    double* x;
+    ulonglong2* ex;            // 2 x n exchange slots {value, sequence number}
+    unsigned long long seq;    // sequence numbers of this solve start above this
+    DevScalars* sc;            // results: iterations, residual norms, convergence; the error word
+    long long wait_limit;      // bound of each exchange wait, SM clock cycles
+};
+
+__device__ __forceinline__ void slot_store(ulonglong2* p, double v, unsigned long long seq) {
+    asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(seq)
+                 : "memory");
+}
+__device__ __forceinline__ void slot_load(const ulonglong2* p, unsigned long long& v, unsigned long long& seq) {
+    asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+                 : "=l"(v), "=l"(seq)
+                 : "l"(p)
+                 : "memory");
+}
+
+// Two sums over the CTA's threads, the same bits in every thread and, from the same inputs, in every
+// CTA; false when some thread's exchange wait expired (!ok).  rs: 2 RB_WARPS doubles, written again only
+// after another barrier of the CTA.
+__device__ __forceinline__ bool cta_sums(double* rs, double u, double w, bool ok, double& su, double& sw) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+        w += __shfl_xor_sync(0xffffffffu, w, o);
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) {
+        rs[wid] = u;
+        rs[RB_WARPS + wid] = w;
+    }
+    const bool bad = __syncthreads_or(!ok);
+    u = rs[lane & (RB_WARPS - 1)];
+    w = rs[RB_WARPS + (lane & (RB_WARPS - 1))];
+#pragma unroll
+    for (int o = RB_WARPS / 2; o > 0; o >>= 1) {
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+        w += __shfl_xor_sync(0xffffffffu, w, o);
+    }
+    su = u;
+    sw = w;
+    return !bad;
+}
+
+// The thread's elements (tid + k RB_T) of the vector published in `slots` under seq.  The warp polls as
+// one: lanes that leave the loop apart would run what follows in as many passes.
+template <int K>
+__device__ __forceinline__ bool collect(const ulonglong2* slots, int n, unsigned long long seq, long long limit,
+                                        int* err, double (&v)[K]) {
+    constexpr int B = K < 4 ? K : 4;  // loads in flight
+    const long long t0 = clock64();
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += B) {
+        unsigned pend = 0;
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            v[k0 + k] = 0.0;
+            if ((int)threadIdx.x + (k0 + k) * RB_T < n) pend |= 1u << k;
+        }
+        while (__any_sync(0xffffffffu, pend)) {
+            unsigned long long lo[B], hi[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if (pend >> k & 1) slot_load(slots + threadIdx.x + (k0 + k) * RB_T, lo[k], hi[k]);
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if ((pend >> k & 1) && hi[k] == seq) {
+                    v[k0 + k] = __longlong_as_double((long long)lo[k]);
+                    pend &= ~(1u << k);
+                }
+            if (__any_sync(0xffffffffu, pend && clock64() - t0 > limit)) {
+                if ((threadIdx.x & 31) == 0) atomicExch(err, 1);
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
+enum { PH_V, PH_T, PH_RX, PH_RT };
+
+template <int K, int M>
+__global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
+    extern __shared__ double smem[];
+    const int n = a.n, np = (n + 1) & ~1, nv = a.nv, tid = threadIdx.x, rows = a.rows;
+    const int row0 = blockIdx.x * rows, nr = min(rows, n - row0), cstep = RB_T / rows;
+    double *vec = smem, *r0 = smem + nv, *invd = r0 + np, *part = invd + np, *red = part + a.npart;
+    double* slab = red + 6 * RB_WARPS;
+    const int i = tid % rows, c = tid / rows;  // the thread's row of the CTA and first column
+    const bool active = c < cstep && i < nr;
+    // the thread's entries of the own rows: columns c + q cstep, the first M in registers, the others
+    // (columns from M cstep on) in shared memory
+    double m[M];
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+        const int j = c + q * cstep;
+        m[q] = active && j < n ? __ldg(a.A + (size_t)j * n + row0 + i) : 0.0;
+    }
+    if (active)
+        for (int j = c + M * cstep; j < n; j += cstep)
+            slab[(j - M * cstep) * rows + i] = __ldg(a.A + (size_t)j * n + row0 + i);
+    for (int e = n + tid; e < nv; e += RB_T) vec[e] = 0.0;  // read with the zero entries past column n
+    // r (s between the two products), p (p - w v after the second), v of the thread's elements
+    double r[K], p[K], v[K];
+    double bb = 0.0, dummy;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int e = tid + k * RB_T;
+        r[k] = p[k] = v[k] = 0.0;
+        if (e < n) {
+            const double d = __ldg(a.A + (size_t)e * n + e), be = __ldg(a.b + e);
+            invd[e] = d != 0.0 ? 1.0 / d : 1.0;
+            r0[e] = be;
+            r[k] = be;
+            bb += be * be;
+        }
+    }
+    cta_sums(red + 4 * RB_WARPS, bb, 0.0, true, bb, dummy);
+    const double tol2 = RB_EPS * RB_EPS * bb;
+    double rr = bb, r0r = bb, r0_sq = bb, rho = 1.0, alpha = 1.0, w = 1.0;
+    double bfac = 1.0;  // (alpha / w) / rho of the iteration before: beta = rho bfac
+    double x = 0.0, y = 0.0;  // of row row0 + tid, tid < nr
+    int iters = 0, restarts = 0, nonconv = 0, phase = PH_V;
+    unsigned long long seq = a.seq;
+    bool begin = bb != 0.0, go = begin;
+    while (go) {
+        if (begin) {  // a new iteration: loop test, then p and y = invd p, or a restart
+            begin = false;
+            if (!(rr > tol2) || iters >= a.maxit) {
+                nonconv = rr > tol2 ? 1 : 0;
+                break;
+            }
+            rho = r0r;
+            phase = fabs(r0r) < RB_EPS * RB_EPS * r0_sq ? PH_RX : PH_V;
+        }
+        ++seq;
+        ulonglong2* slots = a.ex + (size_t)(seq & 1) * n;
+        if (phase == PH_RX) {  // the restart needs all of x
+            if (tid < nr) slot_store(slots + row0 + tid, x, seq);
+        } else {
+            if (phase == PH_V) {
+                const double beta = rho * bfac;
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if (tid + k * RB_T < n) {
+                        p[k] = r[k] + beta * p[k];
+                        vec[tid + k * RB_T] = invd[tid + k * RB_T] * p[k];
+                    }
+            }
+            __syncthreads();
+            // the own rows of A vec
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            if (active) {
+                const double* vc = vec + c;
+#pragma unroll
+                for (int q = 0; q < M; ++q) acc[q & 3] = fma(m[q], vc[q * cstep], acc[q & 3]);
+                int j = c + M * cstep;
+                const double* sl = slab + c * rows + i;
+                const int sst = cstep * rows;
+                for (; j + 3 * cstep < n; j += 4 * cstep, sl += 4 * sst) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[q] = fma(sl[q * sst], vec[j + q * cstep], acc[q]);
+                }
+                for (; j < n; j += cstep, sl += sst) acc[0] = fma(sl[0], vec[j], acc[0]);
+                part[i * (cstep + 1) + c] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+            }
+            __syncthreads();
+            const int lane = tid & 31;
+            for (int q = tid >> 5; q < nr; q += RB_WARPS) {
+                double s = 0.0;
+                for (int k = lane; k < cstep; k += 32) s += part[q * (cstep + 1) + k];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) slot_store(slots + row0 + q, s, seq);
+            }
+            if (phase == PH_V && tid < nr) y = vec[row0 + tid];
+        }
+        double t[K];
+        const bool ok = collect<K>(slots, n, seq, a.wait_limit, &a.sc->wait_err, t);
+        if (phase == PH_V) {
+            double s0 = 0.0, r0v;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                v[k] = t[k];
+                if (tid + k * RB_T < n) s0 += r0[tid + k * RB_T] * v[k];
+            }
+            if (!cta_sums(red, s0, 0.0, ok, r0v, dummy)) return;
+            alpha = rho / r0v;
+            // s = r - alpha v; z = invd s
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (tid + k * RB_T < n) {
+                    r[k] = r[k] - alpha * v[k];
+                    vec[tid + k * RB_T] = invd[tid + k * RB_T] * r[k];
+                }
+            phase = PH_T;
+        } else if (phase == PH_T) {
+            const double z = tid < nr ? vec[row0 + tid] : 0.0;
+            double s0 = 0.0, s1 = 0.0, tt, ts;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                s0 += t[k] * t[k];
+                s1 += t[k] * r[k];
+            }
+            if (!cta_sums(red + 2 * RB_WARPS, s0, s1, ok, tt, ts)) return;
+            w = tt > 0.0 ? ts / tt : 0.0;
+            bfac = (alpha / w) / rho;
+            x += alpha * y + w * z;
+            s0 = s1 = 0.0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                r[k] = r[k] - w * t[k];
+                p[k] = p[k] - w * v[k];
+                s0 += r[k] * r[k];
+                if (tid + k * RB_T < n) s1 += r0[tid + k * RB_T] * r[k];
+            }
+            cta_sums(red + 4 * RB_WARPS, s0, s1, true, rr, r0r);
+            ++iters;
+            begin = true;
+        } else if (phase == PH_RX) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (tid + k * RB_T < n) vec[tid + k * RB_T] = t[k];
+            if (__syncthreads_or(!ok)) return;
+            phase = PH_RT;
+        } else {  // r = b - A x, r0 = r
+            double s0 = 0.0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int e = tid + k * RB_T;
+                if (e < n) {
+                    r[k] = __ldg(a.b + e) - t[k];
+                    r0[e] = r[k];
+                    s0 += r[k] * r[k];
+                }
+            }
+            if (!cta_sums(red, s0, 0.0, ok, rho, dummy)) return;
+            r0_sq = rho;
+            if (restarts++ == 0) iters = 0;
+            phase = PH_V;
+        }
+    }
+    if (tid < nr) a.x[row0 + tid] = x;
+    if (blockIdx.x == 0 && tid == 0) {
+        a.sc->rhs_sq = bb;
+        a.sc->rr = rr;
+        a.sc->iters = iters;
+        a.sc->nonconv = nonconv;
+        a.sc->done = 1;
+    }
+}
+
+template <int K, int M>
+cudaError_t rb_launch(const RBArgs& a, int grid, size_t smem, cudaStream_t s) {
+    static std::atomic<uint64_t> ready{0};
+    if (!once_per_device(ready, [] {
+            return cudaFuncSetAttribute(k_bicg_resident<K, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
+                   cudaSuccess;
+        }))
+        return cudaErrorUnknown;
+    void* args[] = {const_cast<RBArgs*>(&a)};
+    return cudaLaunchCooperativeKernel((void*)k_bicg_resident<K, M>, grid, RB_T, args, smem, s);
+}
+
+}  // namespace
+
+size_t rbicg_words(int64_t n) { return n <= RB_MAX_N ? 4 * (size_t)n : 0; }
+
+int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s) {
+    const int n = (int)c.topo.N;
+    const int maxit = c.prm.max_iters > 0 ? c.prm.max_iters : 2 * n;
+    int sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.device);
+    if (!coop || n > RB_MAX_N || maxit > 4 * RB_MAX_N) return BEM_ERR_STATE;
+    RBArgs a{};
+    a.n = n;
+    a.rows = std::max(std::min(n, 16), (n + sms - 1) / sms);
+    const int grid = (n + a.rows - 1) / a.rows, np = (n + 1) & ~1, cstep = RB_T / a.rows;
+    const int K = (n + RB_T - 1) / RB_T;
+    const int M = K == 1 ? (n <= 8 * cstep ? 8 : 16) : K == 2 ? 28 : K == 3 ? 24 : 20;
+    a.nv = std::max(np, M * cstep);
+    a.nv += a.nv & 1;
+    a.npart = a.rows * (cstep + 1);
+    const size_t smem = sizeof(double) * (a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS +
+                                          (size_t)std::max(0, n - M * cstep) * a.rows);
+    if (smem > 227 * 1024) return BEM_ERR_STATE;
+    a.maxit = maxit;
+    a.A = A;
+    a.b = b;
+    a.x = x;
+    a.ex = reinterpret_cast<ulonglong2*>(c.rbicg);
+    a.seq = ++c.rbicg_solves << 32;
+    a.sc = c.sc;
+    a.wait_limit = c.wait_limit;
+    KLAUNCH();
+    const cudaError_t e = K == 1   ? (M == 8 ? rb_launch<1, 8>(a, grid, smem, s) : rb_launch<1, 16>(a, grid, smem, s))
+                          : K == 2 ? rb_launch<2, 28>(a, grid, smem, s)
+                          : K == 3 ? rb_launch<3, 24>(a, grid, smem, s)
+                                   : rb_launch<4, 20>(a, grid, smem, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return BEM_ERR_CUDA;
+    }
+    BEM_CUDA(c, cudaMemcpyAsync(c.h_sc, c.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
+    BEM_CUDA(c, cudaStreamSynchronize(s));
+    if (c.h_sc->wait_err) {
+        BEM_CUDA(c, cudaMemsetAsync(&c.sc->wait_err, 0, sizeof(int32_t), s));
+        c.stats.wait_expired++;
+        return c.fail(BEM_ERR_CUDA, "BiCGSTAB: an exchange wait expired");
+    }
+    c.stats.last_iters = c.h_sc->iters;
+    c.stats.last_rel_residual = c.h_sc->rhs_sq > 0 ? sqrt(c.h_sc->rr / c.h_sc->rhs_sq) : 0.0;
+    c.stats.total_iters += c.stats.last_iters;
+    c.stats.solves++;
+    return BEM_OK;
+}
+
+}  // namespace bemb

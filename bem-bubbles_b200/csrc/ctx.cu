@@ -50,6 +50,7 @@ static void free_all(Ctx& c, bool keep_blocks = false) {
     c.rf_bar = nullptr;
     c.asm_err = nullptr;
     c.pbicg = nullptr;
+    c.rbicg = nullptr;
     c.lu_aux = nullptr;
     c.Xinv = c.Tw = c.G32 = nullptr;
     c.tcp = nullptr;
@@ -699,6 +700,7 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         (rc = dalloc(c, &c.part, (size_t)ncs * n)) || (rc = dalloc(c, &c.cnt, (n + 255) / 256 + 1)) ||
         (rc = dalloc(c, &c.red, (size_t)(c.gmres_m + 8) * VBLK + 4096)) || (rc = dalloc(c, &c.piv, n)) || (rc = dalloc(c, &c.lu_perm, n)) ||
         (rc = dalloc(c, &c.hcol, (size_t)2 * (c.gmres_m + 2) + 8)) || (rc = dalloc(c, &c.pbicg, pbicg_words(N))) ||
+        (!c.batch && (rc = dalloc(c, &c.rbicg, rbicg_words(N)))) ||
         (!c.batch && (rc = dalloc(c, &c.lu_aux, lu_panel_words()))) ||
         (!c.batch && (rc = dalloc(c, &c.psih, (size_t)PRED_DEPTH * 4 * n))) ||
         (!c.batch && (rc = dalloc(c, &c.psih_t, (size_t)PRED_CNT + 1))))
@@ -719,6 +721,7 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         if ((rc = alloc_mixed(c))) return rc;
     }
     BEM_CUDA(c, cudaMemset(c.cnt, 0, sizeof(unsigned) * ((n + 255) / 256 + 1)));
+    if (c.rbicg) BEM_CUDA(c, cudaMemset(c.rbicg, 0, sizeof(double) * rbicg_words(N)));
     BEM_CUDA(c, cudaMemset(c.vol_cnt, 0, sizeof(unsigned) * (size_t)h.nparts));
     BEM_CUDA(c, cudaMemset(c.phi, 0, sizeof(double) * n));
     BEM_CUDA(c, cudaMemset(c.psi, 0, sizeof(double) * n));

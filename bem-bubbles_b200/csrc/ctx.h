@@ -98,6 +98,8 @@ struct Ctx {
     double* Z = nullptr;       // N*m preconditioned directions
     double* hcol = nullptr;    // (m+2) Hessenberg column / dot results
     double* pbicg = nullptr;   // persistent BiCGSTAB: per-row-block dots, barrier and error words
+    double* rbicg = nullptr;   // resident BiCGSTAB: exchange slots (zero at first)
+    unsigned long long rbicg_solves = 0;  // its solves so far (sequence numbers of the slots)
     bool pbicg_ok = true;      // the persistent BiCGSTAB is usable (cleared after a failed launch or wait)
     int* rf_bar = nullptr;     // the mixed solve's round kernel: grid barrier words [0..1], error word [2]
     bool refine_ok = true;     // its cooperative launch is usable (cleared after a failed launch or wait)

@@ -122,7 +122,8 @@ struct DevScalars {
     // BiCGSTAB / GMRES scalars
     double rho, alpha, w, beta, r0_sq, rhs_sq, tol2, rr;
     int32_t iters, restarts, done, restart_flag, maxit, nonconv;
-    int32_t pad[2];
+    int32_t wait_err;  // an exchange wait of the resident BiCGSTAB expired
+    int32_t pad;
 };
 
 // One independent sub-system of a block-diagonal batch (one bubble of a parameter sweep).  Its
@@ -190,6 +191,15 @@ void launch_pin_finish(Ctx& c, const double* x, double* vel, double* pot, cudaSt
 // bicg.cu
 int bicgstab_persistent(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s);
 size_t pbicg_words(int64_t n);  // doubles of the persistent BiCGSTAB's dot and barrier scratch
+
+// bicg_resident.cu
+// Most unknowns of the BiCGSTAB whose vectors stay in registers and shared memory (4 elements of each
+// per thread of 512).
+constexpr int RB_MAX_N = 4 * 512;
+// BEM_OK with the solution in x; BEM_ERR_STATE: not for this size, nothing done; BEM_ERR_CUDA: the
+// launch failed or an exchange wait expired.
+int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s);
+size_t rbicg_words(int64_t n);  // doubles of its exchange slots
 
 // lu_panel.cu
 // The panel of another column-major n x n matrix (only its columns [k0, k0+nb) are touched); piv and

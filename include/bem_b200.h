@@ -286,8 +286,8 @@ typedef struct {
 } bem_stats;
 int bem_get_stats(bem_ctx* ctx, bem_stats* s);
 
-/* Bound, in SM clock cycles, of every grid-wide barrier wait of the persistent kernels (the
- * cooperative BiCGSTAB, the cooperative refinement round, the row-distributed LU panel) and of the
+/* Bound, in SM clock cycles, of every grid-wide barrier or exchange wait of the persistent kernels (the
+ * cooperative BiCGSTAB forms, the cooperative refinement round, the row-distributed LU panel) and of the
  * LU cluster panel's mbarrier waits.  Default 2e9 (about a second at the B200's clock).  A wait that
  * runs out makes the kernel set its error word and return; the host reads it, counts it in
  * bem_stats.wait_expired and finishes the solve with the multi-kernel form (for the LU: the
