@@ -258,276 +258,292 @@ __device__ void lu_build_pairs_warp(int n, int k0, int nb, const int* pj, int* t
 }
 
 // The same panel on one thread-block cluster (up to 16 CTAs), for panels whose rows fit in the
-// cluster's shared memory (about 5700 rows of a 64-column panel).  The candidates travel by push: a
-// column step is
-//   * each thread already holds the largest |entry| of the column among its rows (found while it
-//     eliminated the previous column); one block barrier reduces them to the CTA's candidate;
-//   * warp 0 writes the candidate (|entry|, row, the whole row) into slot `me` of every CTA's inbox,
-//     the CTA owning the diagonal row writes that row into every CTA's diagonal box, and one lane per
-//     destination arrives on the destination's mbarrier (release at cluster scope);
-//   * warp 0 waits (bounded) on its own mbarrier for all CTAs' arrivals (acquire), then picks the
-//     pivot from its inbox: largest |entry|, then smallest row (the single-CTA kernel's rule); the
-//     pivot row and the diagonal row are already in its own shared memory; one block barrier;
-//   * each thread takes its rows: the diagonal row's owner writes the pivot row there, the pivot
-//     row's owner writes the old diagonal row in its place, and every row below the diagonal is
-//     eliminated, l = a_ij * (1 / a_jj), a_ik -= l * a_jk, the next column first, so its candidate
-//     comes with it.
-// Inbox, diagonal box and mbarrier are double-buffered by column parity: a CTA writes column j + 2's
-// candidates only after all CTAs' arrivals for column j + 1, which each CTA makes after it has read
-// its column-j inbox.  A wait that runs out sets *err; the CTA still makes every write and arrival of
-// the remaining columns (so no other CTA waits on it), and the caller factors again without the
-// cluster.
+// cluster's shared memory (about 6300 rows of a 64-column panel).  A thread owns one row: the row sits in
+// shared memory, its entries in the current block of 8 columns in registers.  A column step is
+//   * the largest |entry| of the column over the CTA's rows: one integer warp reduction of the high
+//     words (and of the low words and rows on ties), one block barrier, one more warp reduction;
+//   * every CTA sends its candidate (|entry|, row, reciprocal, the row's 8 block columns) into every
+//     CTA's inbox through distributed shared memory, as 16-byte slots {value, step} written and read as
+//     one access: no fence, no arrival, no second barrier.  Every warp polls (bounded) the inbox of its
+//     own CTA and picks the pivot: largest |entry|, then smallest row;
+//   * each thread eliminates its row in the block's registers, l = a_ij * (1 / a_jj), a_ik -= l a_jk.
+// Rows are not moved: each thread keeps its row's position under the interchanges so far, and writes it
+// there at the end.  The columns right of the block are updated once per block with rank 8, from the
+// pivot rows' entries that their owner sent while the next candidates travelled.  Each entry sees the
+// operations of the column-by-column elimination in the same order.
+// Inboxes alternate by column parity: a CTA sends column j + 2's candidate only after it has read every
+// CTA's for column j + 1, each sent after a block barrier behind the reads of column j.
+// What bounds it: the serial chain of a column step, about 2500 cycles (reductions, barrier, a division,
+// one distributed-shared-memory trip, the share of the rank-8 update).  Measured, mean over a solve's
+// panels: 210 -> 94 us at N = 4002 and 172 -> 84 us at N = 984, against an exchange through mbarrier
+// arrivals and fences by one warp, with the rows interchanged and all columns right of the current one
+// updated in shared memory at every step.
+// A wait that runs out sets *err; the CTA then takes what it finds, makes every send of the remaining
+// columns (so no other CTA waits on it), and the caller factors again without the cluster.
 constexpr int LC_MAX = 16;
 constexpr size_t LC_SMEM = 220 * 1024;  // dynamic shared memory of one cluster CTA, at most
+constexpr int LC_W = 8;                 // columns of a block
+constexpr int LC_SLOTS = 12;            // slots of a candidate: key, row, reciprocal, LC_W entries, pad
+constexpr int LC_REST = LP_NBMAX - LC_W;
 
 __device__ __forceinline__ uint32_t lp_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Bounded wait for phase `parity` of the local mbarrier `bar` (acquire at cluster scope): polls with
-// the non-blocking test_wait and gives up after `limit` SM clock cycles.
-__device__ __forceinline__ bool lp_bar_wait(uint32_t bar, uint32_t parity, long long limit) {
-    const long long t0 = clock64();
-    for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (clock64() - t0 > limit) return false;
-    }
+// 16-byte slot {value, tag} of a CTA's shared memory (a cluster address), one access.
+__device__ __forceinline__ void lc_send(uint32_t addr, unsigned long long v, unsigned long long tag) {
+    asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.cluster.shared::cluster.b128 [%0], q;\n\t}" ::"r"(
+                     addr),
+                 "l"(v), "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ void lc_read(uint32_t addr, unsigned long long& v, unsigned long long& tag) {
+    asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.cluster.shared::cta.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+                 : "=l"(v), "=l"(tag)
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t lc_map(uint32_t addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
 }
 
-// pairs (may be null): CTA 0 also composes the panel's interchanges (lu_build_pairs_warp) at the end.
-__global__ void __launch_bounds__(LP_THREADS) k_lu_panel_cluster(int n, int k0, int nb, int rows_per, double* A,
-                                                                 int* piv, int* sing, int* pairs, int* err,
-                                                                 long long wait_limit) {
+// Lane of the largest key, of the smallest row among equal keys.
+__device__ __forceinline__ int lc_argmax(unsigned long long key, int row) {
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    unsigned m;
+    asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(m) : "r"(hi));
+    bool in = hi == m;
+    unsigned bal = __ballot_sync(0xffffffffu, in);
+    if (bal & (bal - 1)) {
+        asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(m) : "r"(in ? lo : 0u));
+        in = in && lo == m;
+        bal = __ballot_sync(0xffffffffu, in);
+        if (bal & (bal - 1)) {
+            int r;
+            asm volatile("redux.sync.min.s32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(in ? row : 0x7fffffff));
+            bal = __ballot_sync(0xffffffffu, in && row == r);
+        }
+    }
+    return __ffs(bal) - 1;
+}
+
+// pairs (may be null): receives the panel's interchanges as (destination, source) row pairs.
+template <int T>
+__global__ void __launch_bounds__(T) k_lu_panel_cluster(int n, int k0, int nb, int rows_per, double* A, int* piv,
+                                                        int* sing, int* pairs, int* err, long long wait_limit) {
     namespace cgx = cooperative_groups;
+    using u64 = unsigned long long;
     cgx::cluster_group cl = cgx::this_cluster();
-    // dynamic: [rows_per][ld] rows, inbox [2][C][2 + nb], diagonal box [2][nb]
-    extern __shared__ double sp[];
-    constexpr int NW = LP_THREADS / 32;
-    __shared__ double s_v[NW];
-    __shared__ int s_i[NW];
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ double s_rcp;
-    __shared__ int s_p, s_w, s_piv[LP_NBMAX], tab_r[2 * LP_NBMAX], tab_s[2 * LP_NBMAX];
+    constexpr int NW = T / 32, W = LC_W;
+    // dynamic: inbox [2][C][LC_SLOTS], pivot rows [W][LC_REST] as slots; candidates of the warps
+    // [2][NW][LC_SLOTS]; solved pivot rows [LC_REST][W]; multipliers of the pivot rows [W][W]; the rows
+    extern __shared__ __align__(16) unsigned char sraw[];
     const int C = (int)cl.num_blocks(), me = (int)cl.block_rank(), tid = threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
-    const int ld = nb + 1, stride = 2 + nb;
-    double* inbox = sp + (size_t)rows_per * ld;
-    double* dbox = inbox + 2 * C * stride;
-    const int r0 = k0 + me * rows_per, r1 = min(n, r0 + rows_per);
-    const int nr = max(0, r1 - r0);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(lp_smem(&s_bar[0])), "r"(C));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(lp_smem(&s_bar[1])), "r"(C));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    // the CTA's rows of the panel, 16 loads in flight per thread
-    for (int e0 = tid; e0 < nr * nb; e0 += 16 * LP_THREADS) {
-        double v[16];
+    const int ld = nb | 1;
+    ulonglong2* inbox = reinterpret_cast<ulonglong2*>(sraw);
+    ulonglong2* ubox = inbox + 2 * C * LC_SLOTS;
+    u64* cand = reinterpret_cast<u64*>(ubox + W * LC_REST);
+    double* usol = reinterpret_cast<double*>(cand + 2 * NW * LC_SLOTS);
+    double* pl = usol + LC_REST * W;
+    double* sp = pl + W * W;
+    const int r0 = k0 + me * rows_per, nr = max(0, min(n, r0 + rows_per) - r0);
+    const uint32_t inbox_a = lp_smem(inbox), ubox_a = lp_smem(ubox);
+    for (int e = tid; e < 2 * C * LC_SLOTS + W * LC_REST; e += T) inbox[e] = make_ulonglong2(0, 0);
+    if (pairs && me == 0 && tid == 0) pairs[0] = 0;
+    const bool valid = tid < nr;
+    double* row = sp + (size_t)tid * ld;
+    if (valid)
+        for (int c0 = 0; c0 < nb; c0 += 16) {  // 16 loads in flight
+            double v[16];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int e = e0 + u * LP_THREADS, c = e / max(nr, 1), rr = e - c * nr;
-            v[u] = e < nr * nb ? A[(size_t)(k0 + c) * n + r0 + rr] : 0.0;
-        }
+            for (int u = 0; u < 16; ++u) v[u] = c0 + u < nb ? A[(size_t)(k0 + c0 + u) * n + r0 + tid] : 0.0;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int e = e0 + u * LP_THREADS, c = e / max(nr, 1), rr = e - c * nr;
-            if (e < nr * nb) sp[rr * ld + c] = v[u];
+            for (int u = 0; u < 16; ++u)
+                if (c0 + u < nb) row[c0 + u] = v[u];
         }
-    }
-    cl.sync();  // every CTA's mbarriers initialised before anyone arrives on them
-    // this thread's candidate for column 0 (every row of the panel is at or below the diagonal)
-    double best = -1.0;
-    int bi = n;
-    for (int rr = tid; rr < nr; rr += LP_THREADS) {
-        const double v = fabs(sp[rr * ld]);
-        if (v > best) {  // rows increase with rr: the first row wins ties
-            best = v;
-            bi = r0 + rr;
-        }
-    }
-    bool ok = true;
-    for (int j = 0; j < nb; ++j) {
-        const int rowj = k0 + j, par = j & 1;
-        const int owner_j = (rowj - k0) / rows_per;
-        double* box = inbox + (size_t)par * C * stride;  // [C][2 + nb]
-        double* dg = dbox + (size_t)par * nb;
+    cl.sync();  // every CTA's slots are clear before anyone writes into them
+    int pos = valid ? r0 + tid : 0x7fffffff;  // the row's position after the interchanges so far
+    bool active = valid, ok = true;
+    int send_k = -1, send_row = 0;  // the last column's pivot row, if this CTA's: its block step and row
+    for (int jb = 0; jb < nb; jb += W) {
+        const int rest = nb - jb - W;  // columns right of the block
+        double v[W];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) {
-                best = ov;
-                bi = oi;
+        for (int c = 0; c < W; ++c) v[c] = valid && jb + c < nb ? row[jb + c] : 0.0;
+        int kd = -1;  // the block step at which this row became a pivot row
+        // the pivot row of step send_k goes to every CTA, its entries right of the block
+        auto send_pivot_row = [&]() {
+            if (send_k < 0) return;
+            for (int d = wid; d < C; d += NW) {
+                const uint32_t to = lc_map(ubox_a, d) + send_k * LC_REST * 16;
+                for (int c = lane; c < rest; c += 32)
+                    lc_send(to + c * 16, __double_as_longlong(sp[(size_t)send_row * ld + jb + W + c]), jb + send_k + 1);
             }
-        }
-        if (lane == 0) {
-            s_v[wid] = best;
-            s_i[wid] = bi;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            double v = lane < NW ? s_v[lane] : -2.0;
-            int i = lane < NW ? s_i[lane] : n;
+            send_k = -1;
+        };
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-                if (ov > v || (ov == v && oi < i)) {
-                    v = ov;
-                    i = oi;
+        for (int jj = 0; jj < W; ++jj) {
+            const int j = jb + jj;
+            if (j >= nb) break;
+            const int rowj = k0 + j, par = j & 1;
+            const u64 tag = j + 1;
+            u64* mine = cand + (size_t)(par * NW + wid) * LC_SLOTS;
+            // |entry| as an integer, ordered like the value; a NaN is below every number
+            const double av = fabs(v[jj]);
+            u64 key = active && av == av ? (u64)__double_as_longlong(av) + 1 : 0;
+            int kr = active ? pos : 0x7fffffff;
+            const int wl = lc_argmax(key, kr);
+            if (lane == wl) {
+                mine[0] = key;
+                mine[1] = (u64)(unsigned)kr | (u64)(unsigned)tid << 32;
+                mine[2] = __double_as_longlong(v[jj] != 0.0 ? 1.0 / v[jj] : 0.0);
+#pragma unroll
+                for (int c = 0; c < W; ++c) mine[3 + c] = __double_as_longlong(v[c]);
+            }
+            __syncthreads();
+            const u64* wc = cand + (size_t)par * NW * LC_SLOTS;
+            key = lane < NW ? wc[lane * LC_SLOTS] : 0;
+            kr = lane < NW ? (int)wc[lane * LC_SLOTS + 1] : 0x7fffffff;
+            const int ww = lc_argmax(key, kr);
+            const int dest = wid + (lane >> 4) * NW, sl = lane & 15;
+            if (dest < C && sl < 3 + W)
+                lc_send(lc_map(inbox_a, dest) + ((par * C + me) * LC_SLOTS + sl) * 16, wc[ww * LC_SLOTS + sl], tag);
+            send_pivot_row();
+            // every CTA's candidate
+            const uint32_t box = inbox_a + par * C * LC_SLOTS * 16;
+            u64 a0 = 0, a1 = 0x7fffffff, t0, t1;
+            long long tw = 0;
+            for (;;) {
+                bool have = true;
+                if (lane < C) {
+                    lc_read(box + lane * LC_SLOTS * 16, a0, t0);
+                    lc_read(box + lane * LC_SLOTS * 16 + 16, a1, t1);
+                    have = t0 == tag && t1 == tag;
+                }
+                if (__all_sync(0xffffffffu, have)) break;
+                const long long now = clock64();
+                if (!tw) tw = now;
+                if (__any_sync(0xffffffffu, !ok || now - tw >= wait_limit)) {
+                    ok = false;
+                    if (!have) {
+                        a0 = 0;
+                        a1 = 0x7fffffff;
+                    }
+                    break;
                 }
             }
-            // the candidate row (two columns per lane) and, from the owner, the diagonal row
-            const bool h0 = lane < nb, h1 = lane + 32 < nb;
-            const double* crow = sp + (size_t)(i < n ? i - r0 : 0) * ld;
-            const double c0v = (i < n && h0) ? crow[lane] : 0.0, c1v = (i < n && h1) ? crow[lane + 32] : 0.0;
-            const bool own = me == owner_j;
-            const double* drow_l = sp + (size_t)(own ? rowj - r0 : 0) * ld;
-            const double d0v = (own && h0) ? drow_l[lane] : 0.0, d1v = (own && h1) ? drow_l[lane + 32] : 0.0;
-            double* slot = box + (size_t)me * stride;
-            for (int t = 0; t < C; ++t) {
-                double* rs = cl.map_shared_rank(slot, t);
-                if (lane == 0) {
-                    rs[0] = v;
-                    rs[1] = (double)i;
-                }
-                if (h0) rs[2 + lane] = c0v;
-                if (h1) rs[2 + lane + 32] = c1v;
-                if (own) {
-                    double* rd = cl.map_shared_rank(dg, t);
-                    if (h0) rd[lane] = d0v;
-                    if (h1) rd[lane + 32] = d1v;
-                }
-            }
-            asm volatile("fence.acq_rel.cluster;" ::: "memory");
-            __syncwarp();
-            if (lane < C) {
-                uint32_t rb;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(lp_smem(&s_bar[par])), "r"(lane));
-                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(rb) : "memory");
-            }
-            // all CTAs' candidates for this column, then the pivot (the same in every CTA)
-            if (!lp_bar_wait(lp_smem(&s_bar[par]), (uint32_t)((j >> 1) & 1), wait_limit)) ok = false;
-            double bv = -1.0;
-            int bi2 = n, bw = -1;
-            if (lane < C) {
-                const double* rc = box + (size_t)lane * stride;
-                const int ri = (int)rc[1];
-                if (ri < n) {
-                    bv = rc[0];
-                    bi2 = ri;
-                    bw = lane;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi2, o);
-                const int ow = __shfl_xor_sync(0xffffffffu, bw, o);
-                if (oi < n && (ov > bv || (ov == bv && oi < bi2))) {
-                    bv = ov;
-                    bi2 = oi;
-                    bw = ow;
-                }
-            }
-            if (bw >= 0 && (bi2 < rowj || bi2 >= n)) {  // not a row of this column's candidates: only
-                bw = -1;                                // after an expired wait (garbage), never used
-                bi2 = n;
+            const int w = lc_argmax(a0, (int)a1);
+            int p = (int)__shfl_sync(0xffffffffu, (unsigned)a1, w);
+            const int prow = (int)__shfl_sync(0xffffffffu, (unsigned)(a1 >> 32), w);
+            if (p < rowj || p >= n) {  // only after an expired wait: keep every index in range
+                p = rowj;
                 ok = false;
             }
-            if (lane == 0) {
-                const int p = (bi2 < n) ? bi2 : rowj;  // no candidate: keep the diagonal row
-                const double d = (bw >= 0) ? box[(size_t)bw * stride + 2 + j] : dg[j];
-                s_p = p;
-                s_w = bw;
-                s_rcp = d != 0.0 ? 1.0 / d : 0.0;
-                s_piv[j] = p;
+            // its reciprocal and block entries, and (warp 0) its earlier multipliers for the rank-8 update
+            double u[W], rcp;
+            const uint32_t ws = box + min(w, C - 1) * LC_SLOTS * 16;
+            for (;;) {
+                u64 tags[W + 1], x;
+                lc_read(ws + 32, x, tags[W]);
+                rcp = __longlong_as_double(x);
+                bool have = tags[W] == tag;
+#pragma unroll
+                for (int c = 0; c < W; ++c) {
+                    lc_read(ws + 48 + c * 16, x, tags[c]);
+                    u[c] = __longlong_as_double(x);
+                    have = have && tags[c] == tag;
+                }
+                if (have || !ok) break;
+                const long long now = clock64();
+                if (!tw) tw = now;
+                if (now - tw >= wait_limit) ok = false;
+            }
+            if (tid == 0) {
+#pragma unroll
+                for (int c = 0; c < jj; ++c) pl[jj * W + c] = u[c];
                 if (me == 0) {
                     piv[rowj] = p;
-                    if (d == 0.0) *sing = 1;
+                    if (u[jj] == 0.0) *sing = 1;
                 }
+            }
+            if (active) {
+                if (pos == p) {
+                    active = false;
+                    kd = jj;
+                    pos = rowj;
+                } else {
+                    if (pos == rowj) pos = p;
+                    double l = v[jj];
+                    if (rcp != 0.0) l *= rcp;
+                    v[jj] = l;
+#pragma unroll
+                    for (int c = jj + 1; c < W; ++c) v[c] -= l * u[c];
+                }
+            }
+            if (w == me && rest > 0) {
+                send_k = jj;
+                send_row = min(prow, nr - 1);
+            }
+        }
+        if (valid && (active || kd >= 0)) {
+#pragma unroll
+            for (int c = 0; c < W; ++c)
+                if (jb + c < nb) row[jb + c] = v[c];
+        }
+        if (rest <= 0) continue;
+        send_pivot_row();
+        __syncthreads();  // the pivot rows' multipliers
+        if (tid < rest) {
+            // column jb + W + tid of the block's pivot rows, each less the pivot rows before it
+            double u[W];
+            long long tw = 0;
+            for (;;) {
+                bool have = true;
+#pragma unroll
+                for (int k = 0; k < W; ++k) {
+                    u64 x, t;
+                    lc_read(ubox_a + (k * LC_REST + tid) * 16, x, t);
+                    u[k] = __longlong_as_double(x);
+                    have = have && t == (u64)(jb + k + 1);
+                }
+                if (have || !ok) break;
+                const long long now = clock64();
+                if (!tw) tw = now;
+                if (now - tw >= wait_limit) ok = false;
+            }
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+#pragma unroll
+                for (int i = 0; i < k; ++i) u[k] -= pl[k * W + i] * u[i];
+                usol[tid * W + k] = u[k];
             }
         }
         __syncthreads();
-        const int p = s_p, w = s_w;
-        const double rcp = s_rcp;
-        const double* prow = (w >= 0) ? box + (size_t)w * stride + 2 : dg;
-        best = -1.0;
-        bi = n;
-        for (int rr = tid; rr < nr; rr += LP_THREADS) {
-            const int i = r0 + rr;
-            if (i < rowj) continue;
-            double* row = sp + rr * ld;
-            // copies and updates go eight columns at a time, their loads before their stores (one
-            // column at a time each load waits behind the previous store: the warp of the one lane
-            // doing it then holds up the column step)
-            if (i == rowj) {  // the pivot row moves here, multipliers of the earlier columns included
-                if (p != rowj)
-                    for (int cb = 0; cb < nb; cb += 8) {
-                        double pv[8];
+        if (active) {
+#pragma unroll 4
+            for (int c = 0; c < rest; ++c) {
+                double x = row[jb + W + c];
 #pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            if (cb + u < nb) pv[u] = prow[cb + u];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            if (cb + u < nb) row[cb + u] = pv[u];
-                    }
-                continue;
+                for (int k = 0; k < W; ++k) x -= v[k] * usol[c * W + k];
+                row[jb + W + c] = x;
             }
-            // the old diagonal row moves to the pivot's place: its earlier multipliers are copied and
-            // the rest is eliminated straight from the diagonal box
-            const double* src = row;
-            if (i == p) {
-                src = dg;
-                for (int cb = 0; cb < j; cb += 8) {
-                    double dv[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (cb + u < j) dv[u] = dg[cb + u];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (cb + u < j) row[cb + u] = dv[u];
-                }
-            }
-            double l = src[j];
-            if (rcp != 0.0) l *= rcp;
-            row[j] = l;
-            if (j + 1 < nb) {
-                const double v1 = src[j + 1] - l * prow[j + 1];
-                row[j + 1] = v1;
-                const double a1 = fabs(v1);
-                if (a1 > best) {  // rows increase with rr
-                    best = a1;
-                    bi = i;
-                }
-            }
-            for (int cb = j + 2; cb < nb; cb += 8) {
-                double rv[8], pv[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (cb + u < nb) {
-                        rv[u] = src[cb + u];
-                        pv[u] = prow[cb + u];
-                    }
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (cb + u < nb) row[cb + u] = rv[u] - l * pv[u];
+        } else if (kd >= 0) {
+            for (int c = 0; c < rest; ++c) row[jb + W + c] = usol[c * W + kd];
+        }
+    }
+    if (__any_sync(0xffffffffu, !ok) && lane == 0) atomicExch(err, 1);
+    cl.sync();  // no CTA leaves while another may still write into its shared memory
+    if (valid && pos < n) {
+        for (int c = 0; c < nb; ++c) A[(size_t)(k0 + c) * n + pos] = row[c];
+        if (pairs && pos != r0 + tid) {
+            const int k = atomicAdd(pairs, 1);
+            if (k < 2 * LP_NBMAX) {
+                pairs[1 + 2 * k] = pos;
+                pairs[2 + 2 * k] = r0 + tid;
             }
         }
     }
-    if (!ok && lane == 0) atomicExch(err, 1);
-    cl.sync();  // no CTA leaves while another may still write into its shared memory
-    for (int e = tid; e < nr * nb; e += LP_THREADS) {
-        const int c = e / nr, rr = e - c * nr;
-        A[(size_t)(k0 + c) * n + r0 + rr] = sp[rr * ld + c];
-    }
-    if (pairs && me == 0 && wid == 0) lu_build_pairs_warp(n, k0, nb, s_piv, tab_r, tab_s, pairs);
 }
 
 // Row interchanges of a panel applied to the columns outside it, as one permutation: the panel's
@@ -543,7 +559,7 @@ __global__ void __launch_bounds__(32) k_lu_perm_build(int n, int k0, int nb, con
 __global__ void k_lu_perm_apply(int n, int k0, int nb, const int* __restrict__ pairs, double* __restrict__ A,
                                 int* __restrict__ perm) {
     const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int m = pairs[0];
+    const int m = min(pairs[0], 2 * LP_NBMAX);  // more only after an expired wait in the panel
     constexpr int NQ = (2 * LP_NBMAX + 31) / 32;
     if (col == n && perm) {
         int v[NQ];
@@ -605,24 +621,17 @@ void lu_perm_init(Ctx& c, cudaStream_t s) {
     KLAUNCH(), k_iota_int<<<(n + 255) / 256, 256, 0, s>>>(n, c.lu_perm);
 }
 
-// The panel on one thread-block cluster when its rows fit; BEM_ERR_CUDA when they do not or the
-// cluster launch is unavailable.
-int lu_panel_cluster(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* tgt) {
-    const int n = tgt ? tgt->n : (int)c.topo.N;
-    double* A = tgt ? tgt->A : c.LU;
-    int* piv = tgt ? tgt->piv : c.piv;
-    int* sing = tgt ? tgt->sing : c.flag;
-    const int P = n - k0;
-    if (nb > LP_NBMAX) return BEM_ERR_CUDA;
-    const int C = std::max(1, std::min(LC_MAX, (P + 127) / 128));
-    const int rows_per = (P + C - 1) / C;
-    const size_t smem = sizeof(double) * ((size_t)rows_per * (nb + 1) + (size_t)2 * C * (2 + nb) + 2 * nb);
+template <int T>
+static int launch_panel_cluster(Ctx& c, int n, int k0, int nb, int C, int rows_per, double* A, int* piv, int* sing,
+                                bool want_pairs, cudaStream_t s) {
+    const size_t smem = 16 * ((size_t)2 * C * LC_SLOTS + LC_W * LC_REST) +
+                        8 * ((size_t)2 * (T / 32) * LC_SLOTS + LC_REST * LC_W + LC_W * LC_W + (size_t)rows_per * (nb | 1));
     if (smem > LC_SMEM) return BEM_ERR_CUDA;
     static std::atomic<uint64_t> attr{0};
     if (!once_per_device(attr, [] {
-            return cudaFuncSetAttribute(k_lu_panel_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LC_SMEM) ==
-                       cudaSuccess &&
-                   cudaFuncSetAttribute(k_lu_panel_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            return cudaFuncSetAttribute(k_lu_panel_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)LC_SMEM) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_lu_panel_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
                        cudaSuccess;
         })) {
         cudaGetLastError();
@@ -630,7 +639,7 @@ int lu_panel_cluster(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(LP_THREADS);
+    cfg.blockDim = dim3(T);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -641,18 +650,36 @@ int lu_panel_cluster(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* 
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k_lu_panel_cluster, &cfg) != cudaSuccess || clusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_lu_panel_cluster<T>, &cfg) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
         return BEM_ERR_CUDA;
     }
     KLAUNCH();
-    int* pairs = tgt ? nullptr : lp_pairs(c);  // the interchange pairs of c.LU's panel, composed in the kernel
-    if (cudaLaunchKernelEx(&cfg, k_lu_panel_cluster, n, k0, nb, rows_per, A, piv, sing, pairs, lu_panel_err(c),
+    int* pairs = want_pairs ? lp_pairs(c) : nullptr;  // the interchange pairs of c.LU's panel
+    if (cudaLaunchKernelEx(&cfg, k_lu_panel_cluster<T>, n, k0, nb, rows_per, A, piv, sing, pairs, lu_panel_err(c),
                            (long long)c.wait_limit) != cudaSuccess) {
         cudaGetLastError();
         return BEM_ERR_CUDA;
     }
     return BEM_OK;
+}
+
+// The panel on one thread-block cluster when its rows fit; BEM_ERR_CUDA when they do not or the
+// cluster launch is unavailable.
+int lu_panel_cluster(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* tgt) {
+    const int n = tgt ? tgt->n : (int)c.topo.N;
+    double* A = tgt ? tgt->A : c.LU;
+    int* piv = tgt ? tgt->piv : c.piv;
+    int* sing = tgt ? tgt->sing : c.flag;
+    const int P = n - k0;
+    if (nb > LP_NBMAX) return BEM_ERR_CUDA;
+    // one row per thread; as few CTAs as hold the rows with 256 threads each (512 above 16 x 256 rows):
+    // the exchange's cost grows little with the CTAs, but none of them does any work in it
+    const int C = std::max(1, std::min(LC_MAX, (P + 255) / 256));
+    const int rows_per = (P + C - 1) / C;
+    if (rows_per > 512) return BEM_ERR_CUDA;
+    return rows_per <= 256 ? launch_panel_cluster<256>(c, n, k0, nb, C, rows_per, A, piv, sing, tgt == nullptr, s)
+                           : launch_panel_cluster<512>(c, n, k0, nb, C, rows_per, A, piv, sing, tgt == nullptr, s);
 }
 
 int* lu_panel_err(Ctx& c) { return reinterpret_cast<int*>(lp_bar(c) + 2); }

@@ -288,7 +288,7 @@ int bem_get_stats(bem_ctx* ctx, bem_stats* s);
 
 /* Bound, in SM clock cycles, of every grid-wide barrier or exchange wait of the persistent kernels (the
  * cooperative BiCGSTAB forms, the cooperative refinement round, the row-distributed LU panel) and of the
- * LU cluster panel's mbarrier waits.  Default 2e9 (about a second at the B200's clock).  A wait that
+ * LU cluster panel's exchange waits.  Default 2e9 (about a second at the B200's clock).  A wait that
  * runs out makes the kernel set its error word and return; the host reads it, counts it in
  * bem_stats.wait_expired and finishes the solve with the multi-kernel form (for the LU: the
  * single-CTA panel), which the context keeps for the rest of its life.  No counterpart in the reference (its solves
