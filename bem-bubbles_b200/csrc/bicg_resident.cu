@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "ctx.h"
+#include "slots.cuh"
 
 namespace bemb {
 
@@ -50,18 +51,6 @@ struct RBArgs {
     DevScalars* sc;            // results: iterations, residual norms, convergence; the error word
     long long wait_limit;      // bound of each exchange wait, SM clock cycles
 };
-
-__device__ __forceinline__ void slot_store(ulonglong2* p, double v, unsigned long long seq) {
-    asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
-                 "l"(__double_as_longlong(v)), "l"(seq)
-                 : "memory");
-}
-__device__ __forceinline__ void slot_load(const ulonglong2* p, unsigned long long& v, unsigned long long& seq) {
-    asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
-                 : "=l"(v), "=l"(seq)
-                 : "l"(p)
-                 : "memory");
-}
 
 // Two sums over the CTA's threads, the same bits in every thread and, from the same inputs, in every
 // CTA; false when some thread's exchange wait expired (!ok).  rs: 2 RB_WARPS doubles, written again only

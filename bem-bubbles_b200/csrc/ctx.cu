@@ -692,13 +692,13 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
                        &c.kp3, &c.kp4, &c.r, &c.r0, &c.pv, &c.vv, &c.yv, &c.zv, &c.sv, &c.tv, &c.invd, &c.potz};
     for (auto p : vecs)
         if ((rc = dalloc(c, p, n))) return rc;
-    if ((rc = dalloc(c, &c.G, nn)) || (rc = dalloc(c, &c.H, nn)) || (!c.batch && (rc = dalloc(c, &c.LU, nn))) ||
+    if ((rc = dalloc(c, &c.G, nn)) || (rc = dalloc(c, &c.H, nn)) || (!c.batch && (rc = dalloc(c, &c.LU, nn + n))) ||
         (rc = dalloc(c, &c.rec, m * REC)) || (rc = dalloc(c, &c.tn, 3 * m)) || (rc = dalloc(c, &c.tg, 3 * m)) ||
         (rc = dalloc(c, &c.tk, m)) || (rc = dalloc(c, &c.rowHp, nrow_part)) ||
         (rc = dalloc(c, &c.bp, nrow_part)) || (!c.batch && (rc = dalloc(c, &c.gp, nrow_part))) || (rc = dalloc(c, &c.vol, (size_t)h.nparts + 1)) ||
         (rc = dalloc(c, &c.vol_part, (size_t)h.nparts * 64)) || (rc = dalloc(c, &c.vol_cnt, (size_t)h.nparts)) ||
         (rc = dalloc(c, &c.part, (size_t)ncs * n)) || (rc = dalloc(c, &c.cnt, (n + 255) / 256 + 1)) ||
-        (rc = dalloc(c, &c.red, (size_t)(c.gmres_m + 8) * VBLK + 4096)) || (rc = dalloc(c, &c.piv, n)) || (rc = dalloc(c, &c.lu_perm, n)) ||
+        (rc = dalloc(c, &c.red, (size_t)(c.gmres_m + 8) * VBLK + 4096)) || (rc = dalloc(c, &c.piv, n)) || (!c.batch && (rc = dalloc(c, &c.lu_x, 2 * n))) ||
         (rc = dalloc(c, &c.hcol, (size_t)2 * (c.gmres_m + 2) + 8)) || (rc = dalloc(c, &c.pbicg, pbicg_words(N))) ||
         (!c.batch && (rc = dalloc(c, &c.rbicg, rbicg_words(N)))) ||
         (!c.batch && (rc = dalloc(c, &c.lu_aux, lu_panel_words()))) ||
@@ -721,6 +721,7 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         if ((rc = alloc_mixed(c))) return rc;
     }
     BEM_CUDA(c, cudaMemset(c.cnt, 0, sizeof(unsigned) * ((n + 255) / 256 + 1)));
+    if (c.lu_x) BEM_CUDA(c, cudaMemset(c.lu_x, 0, sizeof(double) * 2 * n));
     if (c.rbicg) BEM_CUDA(c, cudaMemset(c.rbicg, 0, sizeof(double) * rbicg_words(N)));
     BEM_CUDA(c, cudaMemset(c.vol_cnt, 0, sizeof(unsigned) * (size_t)h.nparts));
     BEM_CUDA(c, cudaMemset(c.phi, 0, sizeof(double) * n));
@@ -783,6 +784,7 @@ int bem_create(bem_ctx** out, int device, const bem_params* p) {
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void**)&c->sc, sizeof(DevScalars)) != cudaSuccess ||
         cudaMallocHost((void**)&c->h_sc, sizeof(DevScalars)) != cudaSuccess ||
+        cudaMallocHost((void**)&c->h_flag, 2 * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void**)&c->flag, 4 * sizeof(int)) != cudaSuccess) {
         delete c;
         return BEM_ERR_CUDA;
@@ -808,6 +810,7 @@ int bem_destroy(bem_ctx* c) {
     cudaFree(c->sc);
     cudaFree(c->flag);
     cudaFreeHost(c->h_sc);
+    cudaFreeHost(c->h_flag);
     cudaFreeHost(c->h_red);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;

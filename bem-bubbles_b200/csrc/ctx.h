@@ -45,6 +45,7 @@ struct Ctx {
     double* psi = nullptr;  // N
     DevScalars* sc = nullptr;
     DevScalars* h_sc = nullptr;  // pinned mirror
+    int* h_flag = nullptr;       // pinned: the LU's error words
     double* h_red = nullptr;     // pinned host copy of the mixed solve's residual-norm partials
     size_t h_red_cap = 0;        // its capacity in doubles
 
@@ -80,9 +81,11 @@ struct Ctx {
     double *r = nullptr, *r0 = nullptr, *pv = nullptr, *vv = nullptr, *yv = nullptr, *zv = nullptr,
            *sv = nullptr, *tv = nullptr, *invd = nullptr;
     // LU
-    double* LU = nullptr;  // N*N
+    double* LU = nullptr;  // N*(N+1): the matrix with the right-hand side as column N
     int* piv = nullptr;    // N
-    int* lu_perm = nullptr;  // N: the factorisation's composed row permutation (row i of P A is row lu_perm[i])
+    double* lu_x = nullptr;  // back substitution: N exchange slots of 16 bytes (zero at first)
+    unsigned long long lu_solves = 0;  // its sequence numbers so far
+    bool lu_back_ok = true;    // its cooperative launch is usable (cleared after a failed launch or wait)
     // the LU's look-ahead: the next panel on a high-priority stream beside the current trailing update
     cudaStream_t lu_side = nullptr;
     cudaEvent_t lu_ev[2] = {nullptr, nullptr};

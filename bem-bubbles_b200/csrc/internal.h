@@ -212,10 +212,10 @@ struct PanelTarget {
 };
 int lu_panel_rows(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* tgt = nullptr);
 int lu_panel_cluster(Ctx& c, int k0, int nb, cudaStream_t s, const PanelTarget* tgt = nullptr);
-// the panel's interchanges on the other columns of c.LU and on c.lu_perm; built: the (cluster) panel
-// kernel composed them already
-void lu_panel_swap_rest(Ctx& c, int k0, int nb, cudaStream_t s, bool built);
-void lu_perm_init(Ctx& c, cudaStream_t s);  // c.lu_perm = identity, before the first panel
+// The interchanges of c.LU's last panel as (destination, source) row pairs on the device: their number,
+// then the pairs; at most 2 x 64 of them.  built: the (cluster) panel kernel composed them already.
+constexpr int LU_MAX_PAIRS = 128;
+const int* lu_panel_pairs(Ctx& c, int k0, int nb, cudaStream_t s, bool built);
 // lu_update.cu: A22 -= L21 U12 after the panel [k0, k0 + nb) of the column-major n x n A (FP64 tensor cores)
 int lu_update(Ctx& c, int n, int k0, int nb, double* A, cudaStream_t s, int cb = -1, int ce = -1, bool narrow = false);
 size_t lu_panel_words();   // doubles of Ctx::lu_aux

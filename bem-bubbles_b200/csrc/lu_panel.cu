@@ -546,55 +546,12 @@ __global__ void __launch_bounds__(T) k_lu_panel_cluster(int n, int k0, int nb, i
     }
 }
 
-// Row interchanges of a panel applied to the columns outside it, as one permutation: the panel's
-// transpositions (k0 + j, pj[j]) composed into (destination, source) row pairs by one warp, then one
-// warp per column loads every source before storing any destination.
+// The panel's transpositions (k0 + j, pj[j]) composed into (destination, source) row pairs by one warp;
+// k_lu_swap_trsm (linalg.cu) applies them.
 __global__ void __launch_bounds__(32) k_lu_perm_build(int n, int k0, int nb, const int* __restrict__ piv,
                                                       int* __restrict__ pairs) {
     __shared__ int tab_r[2 * LP_NBMAX], tab_s[2 * LP_NBMAX];
     lu_build_pairs_warp(n, k0, nb, piv + k0, tab_r, tab_s, pairs);
-}
-
-// perm (may be null): the composed row permutation so far, permuted like one more column
-__global__ void k_lu_perm_apply(int n, int k0, int nb, const int* __restrict__ pairs, double* __restrict__ A,
-                                int* __restrict__ perm) {
-    const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int m = min(pairs[0], 2 * LP_NBMAX);  // more only after an expired wait in the panel
-    constexpr int NQ = (2 * LP_NBMAX + 31) / 32;
-    if (col == n && perm) {
-        int v[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int k = lane + 32 * q;
-            if (k < m) v[q] = perm[pairs[2 + 2 * k]];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int k = lane + 32 * q;
-            if (k < m) perm[pairs[1 + 2 * k]] = v[q];
-        }
-        return;
-    }
-    if (col >= n || (col >= k0 && col < k0 + nb)) return;
-    double* a = A + (size_t)col * n;
-    double v[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const int k = lane + 32 * q;
-        if (k < m) v[q] = a[pairs[2 + 2 * k]];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const int k = lane + 32 * q;
-        if (k < m) a[pairs[1 + 2 * k]] = v[q];
-    }
-}
-
-__global__ void k_iota_int(int n, int* __restrict__ v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = i;
 }
 
 }  // namespace
@@ -609,16 +566,10 @@ static int* lp_pairs(Ctx& c) { return reinterpret_cast<int*>(lp_bar(c) + 4); }
 
 size_t lu_panel_words() { return (size_t)2 * LP_GMAX * (2 + LP_NBMAX) + (size_t)2 * LP_NBMAX + 8 + 2 * LP_NBMAX + 8; }
 
-// built: the panel kernel already composed the pairs (the cluster panel of c.LU does)
-void lu_panel_swap_rest(Ctx& c, int k0, int nb, cudaStream_t s, bool built) {
+const int* lu_panel_pairs(Ctx& c, int k0, int nb, cudaStream_t s, bool built) {
     const int n = (int)c.topo.N;
     if (!built) KLAUNCH(), k_lu_perm_build<<<1, 32, 0, s>>>(n, k0, nb, c.piv, lp_pairs(c));
-    KLAUNCH(), k_lu_perm_apply<<<(n + 1 + 7) / 8, 256, 0, s>>>(n, k0, nb, lp_pairs(c), c.LU, c.lu_perm);
-}
-
-void lu_perm_init(Ctx& c, cudaStream_t s) {
-    const int n = (int)c.topo.N;
-    KLAUNCH(), k_iota_int<<<(n + 255) / 256, 256, 0, s>>>(n, c.lu_perm);
+    return lp_pairs(c);
 }
 
 template <int T>
