@@ -204,6 +204,108 @@ __global__ void __launch_bounds__(GV_ROWS) k_gemv(int n, int chunk, const T* __r
     gemv_tile<T, false>(n, chunk, gridDim.y, blockIdx.x, blockIdx.y, A, x, y, part, cnt, u, du, w, dw, cvec, sgn);
 }
 
+// Two consecutive elements of a column, no L2 policy.
+__device__ __forceinline__ void ld_two(const double* p, double& u, double& v) {
+    asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(u), "=d"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_two(const float* p, double& u, double& v) {
+    float a, b;
+    asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
+    u = a;
+    v = b;
+}
+
+// k_gemv for matrices far larger than L2 (gemv_wide has the rule): two rows per thread with one load of
+// two elements per column, and no L2 policy.  The GEMV then only streams: what bounds it is the bytes in
+// flight, and with the policies (which keep X in L2 where it fits) the stream runs at two thirds.  Measured,
+// one FP64 and one FP32 GEMV back to back: n = 32004: 1.93 ms (6.4 TB/s) against 2.80 ms for k_gemv; 15684:
+// 0.47 against 0.66 ms; 10002: 0.21 against 0.28 ms; 5002: 74 against 82 us; 4402: no gain, X begins to stay
+// in L2.  Two rows per thread with the policies, n = 32004: 2.17 ms; one row without them at 10002: 0.33 ms.
+template <typename T>
+__global__ void __launch_bounds__(GV_ROWS) k_gemv_wide(int n, int chunk, const T* __restrict__ A,
+                                                       const double* __restrict__ x, double* y,
+                                                       double* __restrict__ part, unsigned* __restrict__ cnt,
+                                                       const int* __restrict__ gate, int gate_val, const double* u,
+                                                       double* __restrict__ du, const double* w,
+                                                       double* __restrict__ dw, const double* cvec, double sgn) {
+    if (gate && *gate != gate_val) return;
+    const int rb = blockIdx.x, cs = blockIdx.y, ncs = gridDim.y;
+    const int i = rb * 2 * GV_ROWS + 2 * threadIdx.x;  // n is even: rows i and i + 1
+    const int c0 = min(n, cs * chunk), c1 = min(n, c0 + chunk);
+    if (i < n) {
+        double acc0 = 0.0, acc1 = 0.0, bcc0 = 0.0, bcc1 = 0.0;
+        const T* col = A + (size_t)c0 * n + i;
+        int j = c0;
+        for (; j + GV_UNR <= c1; j += GV_UNR) {
+            double a[GV_UNR], b[GV_UNR];
+#pragma unroll
+            for (int q = 0; q < GV_UNR; ++q) ld_two(col + (size_t)q * n, a[q], b[q]);
+#pragma unroll
+            for (int q = 0; q < GV_UNR; q += 2) {
+                const double x0 = __ldg(x + j + q), x1 = __ldg(x + j + q + 1);
+                acc0 = fma(a[q], x0, acc0);
+                bcc0 = fma(b[q], x0, bcc0);
+                acc1 = fma(a[q + 1], x1, acc1);
+                bcc1 = fma(b[q + 1], x1, bcc1);
+            }
+            col += (size_t)GV_UNR * n;
+        }
+        for (; j < c1; ++j) {
+            double a, b;
+            ld_two(col, a, b);
+            acc0 = fma(a, __ldg(x + j), acc0);
+            bcc0 = fma(b, __ldg(x + j), bcc0);
+            col += n;
+        }
+        part[(size_t)cs * n + i] = acc0 + acc1;
+        part[(size_t)cs * n + i + 1] = bcc0 + bcc1;
+    }
+    __threadfence();
+    __shared__ unsigned s_ticket;
+    __syncthreads();
+    if (threadIdx.x == 0) s_ticket = atomicAdd(&cnt[rb], 1u);
+    __syncthreads();
+    if (s_ticket != (unsigned)(ncs - 1)) return;
+    __threadfence();
+    constexpr int PB = 8;
+    double yi[2] = {0.0, 0.0};
+    if (i < n) {
+        int k = 0;
+        for (; k + PB <= ncs; k += PB) {
+            double2 pv[PB];
+#pragma unroll
+            for (int q = 0; q < PB; ++q) pv[q] = __ldcg(reinterpret_cast<const double2*>(part + (size_t)(k + q) * n + i));
+#pragma unroll
+            for (int q = 0; q < PB; ++q) {
+                yi[0] += pv[q].x;
+                yi[1] += pv[q].y;
+            }
+        }
+        for (; k < ncs; ++k) {
+            yi[0] += __ldcg(part + (size_t)k * n + i);
+            yi[1] += __ldcg(part + (size_t)k * n + i + 1);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (cvec) yi[h] = fma(sgn, yi[h], cvec[i + h]);
+            y[i + h] = yi[h];
+        }
+    }
+    // the dots per block of GV_ROWS rows, as k_gemv leaves them: threads below GV_ROWS / 2 hold the first
+    const bool low = threadIdx.x < GV_ROWS / 2;
+    auto dots = [&](const double* z, double* d) {
+        const double v = i < n ? fma(yi[0], z[i], yi[1] * z[i + 1]) : 0.0;
+        const double v0 = block_sum(low ? v : 0.0), v1 = block_sum(low ? 0.0 : v);
+        if (threadIdx.x == 0) {
+            d[2 * rb] = v0;
+            if ((2 * rb + 1) * GV_ROWS < n) d[2 * rb + 1] = v1;
+        }
+    };
+    if (du) dots(u, du);
+    if (dw) dots(w, dw);
+    if (threadIdx.x == 0) cnt[rb] = 0u;
+}
+
 // Column splits: enough CTAs for about eight per SM, at most 64 (the partials buffer holds 64 n).
 static int gemv_splits(int n) {
     const int rb = (n + GV_ROWS - 1) / GV_ROWS;
@@ -212,14 +314,26 @@ static int gemv_splits(int n) {
     return cs;
 }
 
+// k_gemv_wide from about where G and X together (12 n^2 bytes, 265 MB) are twice L2, for even n (two rows
+// per load); four CTAs per SM, eight where every CTA still has many columns (m = 8 against 4 at n = 10002:
+// even; 32004: 2 % faster; 7002: 4 % slower).
+constexpr int GV_WIDE_N = 4700;
+template <typename T>
+static bool gemv_wide(int n, const T* A) {
+    return n >= GV_WIDE_N && n % 2 == 0 && reinterpret_cast<uintptr_t>(A) % (2 * sizeof(T)) == 0;
+}
+
 template <typename T>
 static void gemv_t(int n, const T* A, const double* x, double* y, cudaStream_t s, double* part, unsigned* cnt,
                    const int* gate = nullptr, int gate_val = 0, const double* u = nullptr, double* du = nullptr,
                    const double* w = nullptr, double* dw = nullptr, const double* cvec = nullptr, double sgn = 1.0) {
-    const int ncs = gemv_splits(n);
+    const bool wide = gemv_wide(n, A);
+    const int rows = wide ? 2 * GV_ROWS : GV_ROWS, rb = (n + rows - 1) / rows;
+    const int ncs = wide ? std::max(1, std::min(64, (n < 10000 ? 4 : 8) * 148 / rb)) : gemv_splits(n);
     const int chunk = ((n + ncs - 1) / ncs + GV_UNR - 1) / GV_UNR * GV_UNR;
-    dim3 grid((n + GV_ROWS - 1) / GV_ROWS, ncs);
-    KLAUNCH(), k_gemv<T><<<grid, GV_ROWS, 0, s>>>(n, chunk, A, x, y, part, cnt, gate, gate_val, u, du, w, dw, cvec, sgn);
+    KLAUNCH();
+    (wide ? k_gemv_wide<T> : k_gemv<T>)<<<dim3(rb, ncs), GV_ROWS, 0, s>>>(n, chunk, A, x, y, part, cnt, gate, gate_val,
+                                                                         u, du, w, dw, cvec, sgn);
 }
 
 void gemv(int64_t n, const double* A, const double* x, double* y, cudaStream_t s, double* part, unsigned* cnt) {
