@@ -34,6 +34,8 @@ __constant__ double c_gcos[7], c_gsin[7], c_gw[7];
 //   C + dA * gA_k + dB * gB_k,   C = w0 b0 K(centroid) + cA*S_A + cB*S_B.
 // c_orb = {w0*b0, cA, dA, cB, dB}.
 __constant__ double c_orb[5];
+// The same orbits for the patch kernel: beta and alpha - beta, and the weights of the centroid and the orbits.
+__constant__ double c_pbeta[2], c_pdiff[2], c_pw[3];
 
 // Reference tables (quadrature.hpp:30-38 gauss_7, :88-96 quadrature_7) in the forms the kernels use:
 // per point the basis weights (1-u, u-v, v) * w of the triangle rule applied as (x+y, y) on the
@@ -105,7 +107,17 @@ static void upload_constants() {
     once_per_device(done, [] {
         QuadTables t;
         quad_tables(t);
-        return cudaMemcpyToSymbol(c_orb, t.orb, sizeof(t.orb)) == cudaSuccess &&
+        double pbeta[2], pdiff[2];
+        for (int o = 0; o < 2; ++o) {
+            const double* uv = t.quv[o ? 6 : 3];  // alpha on vertex 0: (alpha, beta, beta)
+            pbeta[o] = uv[1];
+            pdiff[o] = (1.0 - uv[0]) - uv[1];
+        }
+        const double pw[3] = {t.w[0], t.w[3], t.w[6]};
+        return cudaMemcpyToSymbol(c_pbeta, pbeta, sizeof(pbeta)) == cudaSuccess &&
+               cudaMemcpyToSymbol(c_pdiff, pdiff, sizeof(pdiff)) == cudaSuccess &&
+               cudaMemcpyToSymbol(c_pw, pw, sizeof(pw)) == cudaSuccess &&
+               cudaMemcpyToSymbol(c_orb, t.orb, sizeof(t.orb)) == cudaSuccess &&
                cudaMemcpyToSymbol(c_qc, t.qc, sizeof(t.qc)) == cudaSuccess &&
                cudaMemcpyToSymbol(c_quv, t.quv, sizeof(t.quv)) == cudaSuccess &&
                cudaMemcpyToSymbol(c_gcos, t.gc, sizeof(t.gc)) == cudaSuccess &&
@@ -807,13 +819,19 @@ __device__ __forceinline__ bool copy_bar_wait(uint64_t* bar, uint32_t parity, in
 }
 constexpr int COPY_WAIT_POLLS = 1 << 22;  // each poll may suspend the thread for a while: seconds in all
 
-// Patch-order triangle records (PREC doubles): the k_triangle_records layout (0-27), the potential
-// at the three vertices (28-30), the vertex ids (31, 21 bits each, as the bits of a double) and the
-// column slots of the three vertices in the patch (32, 8 bits each).  Without the wall image the
-// image points (16-22) are unused, and those doubles with 33-34 hold the triangle's singular pairs:
-// for row = vertex k of the triangle, the G entry of the column of vertex v at sing_slot(3 k + v).
-// 35 is padding.
-__device__ __forceinline__ int sing_slot(int e) { return e < 7 ? 16 + e : 26 + e; }
+// Patch-order triangle records (PREC doubles), for row distances from the corners: with
+// A = |a - x|^2, B = |b - x|^2 - A = (a - x).2ab + |ab|^2 and C the same for ac, a point y with barycentric
+// weights (l0, l1, l2) lies at |y - x|^2 = A + l1 B + l2 C - W, W = l0 l1 |ab|^2 + l0 l2 |ac|^2 + l1 l2 |bc|^2,
+// so the points of an orbit (weights alpha, beta, beta in turn) share A + beta (B + C).  Layout: the three
+// vertex ids and the column slots (8 bits each) as four ints (0-1); a (2-4), 2ab (5-7), 2ac (8-10), |ab|^2,
+// |ac|^2 (11, 12), -area n (13-15), area (16), -W (17-23) and w phi (24-30) of the points.  The points are the
+// centroid, then the orbits' points by the vertex that has alpha.  Without the wall image 31-39 hold the
+// triangle's singular pairs: for row = vertex k of the triangle, the G entry of the column of vertex v at
+// PR_SING + 3 k + v; with it y.x of the points (31-37).
+constexpr int PR_W = 17, PR_PHI = 24, PR_SING = 31, PR_YX = 31;
+static_assert(PR_SING + 9 <= PREC, "the record holds the singular pairs");
+// the 7-point rule's index (c_quv) of the points in this order
+__constant__ int c_porder[7] = {0, 3, 1, 2, 6, 4, 5};
 
 // Threads [0, M): the records; without the wall image threads [M, 4M) also evaluate the singular
 // pairs, one (triangle, corner) each (Integrator.cpp:13-41), into the record's singular slots.
@@ -829,9 +847,9 @@ __global__ void k_patch_records(int M, const double* __restrict__ x, const doubl
         const int ta = tri[3 * t], tb = tri[3 * t + 1], tc = tri[3 * t + 2];
         double gg[3], hh[3];
         singular_sums<false>(x, ta, tb, tc, k, gg, hh);  // gg[m]: the column of vertex (m + k) % 3
-        double* r = prec + (size_t)p * PREC;
+        double* r = prec + (size_t)p * PREC + PR_SING;
 #pragma unroll
-        for (int m = 0; m < 3; ++m) r[sing_slot(3 * k + (m + k) % 3)] = gg[m];
+        for (int m = 0; m < 3; ++m) r[3 * k + (m + k) % 3] = gg[m];
         return;
     }
     const int p = q;
@@ -840,43 +858,91 @@ __global__ void k_patch_records(int M, const double* __restrict__ x, const doubl
     const int ia = tri[3 * t], ib = tri[3 * t + 1], ic = tri[3 * t + 2];
     const double ax = x[3 * ia], ay = x[3 * ia + 1], az = x[3 * ia + 2];
     const double abx = x[3 * ib] - ax, aby = x[3 * ib + 1] - ay, abz = x[3 * ib + 2] - az;
+    const double acx = x[3 * ic] - ax, acy = x[3 * ic + 1] - ay, acz = x[3 * ic + 2] - az;
     const double bcx = x[3 * ic] - x[3 * ib], bcy = x[3 * ic + 1] - x[3 * ib + 1], bcz = x[3 * ic + 2] - x[3 * ib + 2];
     const double nx = aby * bcz - abz * bcy, ny = abz * bcx - abx * bcz, nz = abx * bcy - aby * bcx;
-    const double area = sqrt(nx * nx + ny * ny + nz * nz);
-    const double ia_ = 1.0 / area;
+    const double ab2 = abx * abx + aby * aby + abz * abz, ac2 = acx * acx + acy * acy + acz * acz;
+    const double bc2 = bcx * bcx + bcy * bcy + bcz * bcz;
     double* r = prec + (size_t)p * PREC;
-    r[0] = ax;
-    r[1] = ay;
-    r[2] = az;
-    r[3] = 2.0 * abx;
-    r[4] = 2.0 * aby;
-    r[5] = 2.0 * abz;
-    r[6] = 2.0 * bcx;
-    r[7] = 2.0 * bcy;
-    r[8] = 2.0 * bcz;
+    *reinterpret_cast<int4*>(r) = make_int4(ia, ib, ic, pslot[p]);
+    r[2] = ax;
+    r[3] = ay;
+    r[4] = az;
+    r[5] = 2.0 * abx;
+    r[6] = 2.0 * aby;
+    r[7] = 2.0 * abz;
+    r[8] = 2.0 * acx;
+    r[9] = 2.0 * acy;
+    r[10] = 2.0 * acz;
+    r[11] = ab2;
+    r[12] = ac2;
+    r[13] = -nx;
+    r[14] = -ny;
+    r[15] = -nz;
+    r[16] = sqrt(nx * nx + ny * ny + nz * nz);
+    const double fa = phi[ia], fb = phi[ib], fc = phi[ic];
 #pragma unroll
-    for (int q2 = 0; q2 < 7; ++q2) {
-        const double u = c_quv[q2][0], v = c_quv[q2][1];
-        const double wx = u * abx + v * bcx, wy = u * aby + v * bcy, wz = u * abz + v * bcz;
-        r[9 + q2] = wx * wx + wy * wy + wz * wz;
-        if (MIRROR) r[16 + q2] = ax + wx;
+    for (int e = 0; e < 7; ++e) {
+        const int k = c_porder[e];
+        const double u = c_quv[k][0], v = c_quv[k][1], l0 = 1.0 - u, l1 = u - v;
+        r[PR_W + e] = -(l0 * l1 * ab2 + l0 * v * ac2 + l1 * v * bc2);
+        r[PR_PHI + e] = c_qc[k][0] * fa + c_qc[k][1] * fb + c_qc[k][2] * fc;
+        if (MIRROR) r[PR_YX + e] = ax + u * abx + v * bcx;
     }
-    const double unx = nx * ia_, uny = ny * ia_, unz = nz * ia_;
-    r[23] = unx;
-    r[24] = uny;
-    r[25] = unz;
-    r[26] = area;
-    r[27] = ax * unx + ay * uny + az * unz;
-    r[28] = phi[ia];
-    r[29] = phi[ib];
-    r[30] = phi[ic];
-    r[31] = __longlong_as_double((long long)ia | ((long long)ib << 21) | ((long long)ic << 42));
-    r[32] = __longlong_as_double((long long)pslot[p]);
-    if (MIRROR) {
-        r[33] = 0.0;
-        r[34] = 0.0;
+}
+
+// One regular (row, triangle) pair: g_k (to be scaled by the area), and hb takes the row's share of b,
+// sum over the points of w (phi(y) - phi_i) * (-area (y - x).n / r^3).  wphi: w phi_i for the three weights.
+// 112 FP64 operations, 49 of them the seven 1/r and 1/r^3.
+template <bool MIRROR>
+__device__ __forceinline__ void patch_pair(const double* __restrict__ rec, double xi0, double xi1, double xi2,
+                                           const double (&wphi)[3], double (&g)[3], double& hb) {
+    // two entries per shared-memory load (the record is 16-byte aligned)
+    double r[MIRROR ? 38 : 32];
+#pragma unroll
+    for (int k = 2; k < (MIRROR ? 38 : 32); k += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(rec + k);
+        r[k] = v.x;
+        r[k + 1] = v.y;
     }
-    r[35] = 0.0;
+    const double ax = r[2] - xi0, ay = r[3] - xi1, az = r[4] - xi2;
+    const double A = fma(ax, ax, fma(ay, ay, __dmul_rn(az, az)));
+    const double B = fma(ax, r[5], fma(ay, r[6], fma(az, r[7], r[11])));
+    const double C = fma(ax, r[8], fma(ay, r[9], fma(az, r[10], r[12])));
+    const double sh = fma(ax, r[13], fma(ay, r[14], __dmul_rn(az, r[15])));  // -area (y - x).n, y in the plane
+    const double BC = B + C;
+    double kg[7], hs = 0.0, hm = 0.0;
+    auto point = [&](int e, double r2, double wp) {
+        const double inv = rsqrt_fp64(r2);
+        const double f = r[PR_PHI + e] - wp;
+        kg[e] = inv;
+        const double inv3 = __dmul_rn(__dmul_rn(inv, inv), inv);
+        hs = e ? fma(inv3, f, hs) : __dmul_rn(inv3, f);
+        if (MIRROR) {
+            // image point (-y.x, y.y, y.z), image normal (-n.x, n.y, n.z) (Integrator.hpp:211-229):
+            // |y' - x|^2 = |y - x|^2 + 4 x.x y.x
+            const double inm = rsqrt_fp64(fma(4.0 * xi0, r[PR_YX + e], r2));
+            kg[e] += inm;
+            const double inm3 = __dmul_rn(__dmul_rn(inm, inm), inm);
+            hm = e ? fma(inm3, f, hm) : __dmul_rn(inm3, f);
+        }
+    };
+    point(0, fma(1.0 / 3.0, BC, A + r[PR_W]), wphi[0]);
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const double P = fma(c_pbeta[o], BC, A);
+        const int e = 1 + 3 * o;
+        point(e, P + r[PR_W + e], wphi[1 + o]);
+        point(e + 1, fma(c_pdiff[o], B, P + r[PR_W + e + 1]), wphi[1 + o]);
+        point(e + 2, fma(c_pdiff[o], C, P + r[PR_W + e + 2]), wphi[1 + o]);
+    }
+    // sum_q w_q basis_k(q) K(q), as orbit_sums
+    const double SA = (kg[2] + kg[3]) + kg[1], SB = (kg[5] + kg[6]) + kg[4];
+    const double K = fma(c_orb[0], kg[0], fma(c_orb[1], SA, __dmul_rn(c_orb[3], SB)));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g[k] = fma(c_orb[2], kg[1 + k], fma(c_orb[4], kg[4 + k], K));
+    hb = fma(hs, sh, hb);
+    if (MIRROR) hb = fma(hm, fma(2.0 * xi0, r[13], sh), hb);  // (y' - x).n' = (a - x).n + 2 x.x n.x
 }
 
 template <int ROWS>
@@ -887,6 +953,13 @@ constexpr size_t patch_smem() {
 // One CTA per tile {patch, first row} of the work list, ROWS rows of the patch's block, one row per
 // thread.  G, the halo columns and the row partials are addressed through the patch's PatchInfo, so
 // the same kernel serves a single system (one block) and a batch of independent bubbles.
+// What bounds it: the pair loop, three quarters of it FP64 issue (N = 4002 without x0: 274 of 300 us, the FP64
+// pipe 66 % active; the finishing sums take 21 us, the column writes 4).  The records read as broadcasts keep
+// the shared-memory pipe at 64 % beside it, so fewer operations per pair gain less than their share: the
+// corner-distance form of the records (112 FP64 operations per pair against 123) took the kernel from 4.61 to
+// 4.44 ms at N = 16002 and from 318 to 309 us at N = 4002.  Measured slower at N = 4002: two rows per thread
+// with half the threads (a record read then serves two rows, 344 us), and a persistent form that defers tickets
+// and finishing sums by a tile (423 us); starting the SM's three CTAs apart changes nothing.
 template <bool MIRROR, int ROWS, int MINB>
 __global__ void __launch_bounds__(ROWS, MINB)
     k_assemble_patch(const int2* __restrict__ work, const PatchInfo* __restrict__ pinfo,
@@ -900,8 +973,9 @@ __global__ void __launch_bounds__(ROWS, MINB)
     double* srec = psmem;                  // [PT_MAX][PREC], the patch's records
     double* acc = psmem + PT_MAX * PREC;   // [PCOLS][ROWS], this CTA's rows of the patch's columns
     __shared__ __align__(8) uint64_t bar;
-    __shared__ int s_col[PCOLS], s_pk[PCOLS];
-    __shared__ long long s_dst[PCOLS];
+    __shared__ int s_pk[PCOLS], s_nc;
+    __shared__ double* s_dst[PCOLS];
+    __shared__ double s_x0[PCOLS];
     const int tid = threadIdx.x;
     const int2 wk = work[blockIdx.x];
     const int p = wk.x;
@@ -911,9 +985,13 @@ __global__ void __launch_bounds__(ROWS, MINB)
     __syncthreads();
     if (tid == 0) bulk_copy_g2s(srec, prec + (size_t)P.t0 * PREC, (uint32_t)(P.nt * PREC * sizeof(double)), &bar);
     if (tid < PCOLS) {
-        s_col[tid] = patch_col[p * PCOLS + tid];
-        s_dst[tid] = patch_dst[p * PCOLS + tid];
+        const int v = patch_col[p * PCOLS + tid];
+        const long long h = patch_dst[p * PCOLS + tid];
+        s_dst[tid] = h < 0 ? G + P.mbase + (long long)(v - P.vbase) * P.n : halo + h;  // where the column goes
         s_pk[tid] = patch_pk[p * PCOLS + tid];
+        const unsigned used = __ballot_sync(0xffffffffu, v >= 0);  // the used slots come first
+        if (tid == 0) s_nc = __popc(used);
+        s_x0[tid] = x0 && v >= 0 ? x0[v] : 0.0;
     }
 #pragma unroll 8
     for (int s = 0; s < PCOLS; ++s) acc[s * ROWS + tid] = 0.0;
@@ -934,45 +1012,42 @@ __global__ void __launch_bounds__(ROWS, MINB)
         }
         return;
     }
-    double hb = 0.0;  // sum over this patch's regular pairs of sum_k H_k (phi_k - phi_i)
+    double hb = 0.0;  // the row's share of b over this patch's regular pairs
+    const double wphi[3] = {__dmul_rn(c_pw[0], phii), __dmul_rn(c_pw[1], phii), __dmul_rn(c_pw[2], phii)};
+    double* mine = acc + tid;
     for (int t = 0; t < (row ? P.nt : 0); ++t) {
         const double* r = srec + t * PREC;
-        const long long ids = __double_as_longlong(r[31]);
-        const int code = (int)__double_as_longlong(r[32]);
-        const int s0 = code & 255, s1 = (code >> 8) & 255, s2 = (code >> 16) & 255;
-        const int ka = i == (int)(ids & 0x1FFFFF) ? 0 : (i == (int)((ids >> 21) & 0x1FFFFF) ? 1 : 2);
-        if (ka < 2 || i == (int)(ids >> 42)) {
+        const int4 id = *reinterpret_cast<const int4*>(r);
+        double* a0 = mine + (id.w & 255) * ROWS;
+        double* a1 = mine + ((id.w >> 8) & 255) * ROWS;
+        double* a2 = mine + ((id.w >> 16) & 255) * ROWS;
+        if (i == id.x || i == id.y || i == id.z) {
             // singular pair: without the wall image its G entries come with the records (the double
             // layer of the flat own triangle vanishes); with it, k_singular_diag<true, true> adds both
             if (!MIRROR) {
-                acc[s0 * ROWS + tid] += r[sing_slot(3 * ka)];
-                acc[s1 * ROWS + tid] += r[sing_slot(3 * ka + 1)];
-                acc[s2 * ROWS + tid] += r[sing_slot(3 * ka + 2)];
+                const double* sg = r + PR_SING + (i == id.x ? 0 : (i == id.y ? 3 : 6));
+                *a0 += sg[0];
+                *a1 += sg[1];
+                *a2 += sg[2];
             }
             continue;
         }
-        PairSums ps;
-        regular_pair<MIRROR>(r, xi0, xi1, xi2, ps);
-        acc[s0 * ROWS + tid] = fma(ps.g[0], ps.area, acc[s0 * ROWS + tid]);
-        acc[s1 * ROWS + tid] = fma(ps.g[1], ps.area, acc[s1 * ROWS + tid]);
-        acc[s2 * ROWS + tid] = fma(ps.g[2], ps.area, acc[s2 * ROWS + tid]);
-        const double e0 = r[28] - phii, e1 = r[29] - phii, e2 = r[30] - phii;
-        hb = fma(fma(ps.h[0], e0, fma(ps.h[1], e1, __dmul_rn(ps.h[2], e2))), ps.sh, hb);
-        if (MIRROR) hb = fma(fma(ps.m[0], e0, fma(ps.m[1], e1, __dmul_rn(ps.m[2], e2))), ps.sm, hb);
+        double g[3];
+        patch_pair<MIRROR>(r, xi0, xi1, xi2, wphi, g, hb);
+        const double area = r[16];
+        *a0 = fma(g[0], area, *a0);
+        *a1 = fma(g[1], area, *a1);
+        *a2 = fma(g[2], area, *a2);
     }
     const int il = i - P.vbase;
     if (row) {
         double gs = 0.0;
-        for (int s = 0; s < PCOLS; ++s) {
-            const int v = s_col[s];
-            if (v < 0) break;
-            const double gv = acc[s * ROWS + tid];
-            const long long h = s_dst[s];
-            if (h < 0)
-                G[P.mbase + (long long)(v - P.vbase) * P.n + il] = gv;
-            else
-                halo[h + il] = gv;
-            if (x0) gs = fma(gv, x0[v], gs);
+        const int nc = s_nc;
+#pragma unroll 4
+        for (int s = 0; s < nc; ++s) s_dst[s][il] = acc[s * ROWS + tid];
+        if (x0) {
+#pragma unroll 4
+            for (int s = 0; s < nc; ++s) gs = fma(acc[s * ROWS + tid], s_x0[s], gs);
         }
         const long long po = P.pbase + (long long)il * P.np + P.lp;  // the row's partials are contiguous
         bp[po] = hb;

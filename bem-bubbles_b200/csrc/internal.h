@@ -50,10 +50,11 @@ constexpr int ASM_TC = 40;
 constexpr int REC = 28;
 // Triangle patches of the G-only assembly (the step path): every triangle belongs to exactly one
 // patch of at most PT_MAX triangles touching at most PCOLS vertices (the patch's columns); a patch
-// record of PREC doubles per triangle (288 bytes, a multiple of 16 for the bulk copy).
+// record of PREC doubles per triangle (320 bytes, a multiple of 16 for the bulk copy; three CTAs' records
+// and accumulators fill an SM's shared memory).
 constexpr int PT_MAX = 32;
 constexpr int PCOLS = 32;
-constexpr int PREC = 36;
+constexpr int PREC = 40;
 constexpr int PATCH_ROWS = 256;  // rows per CTA of the patch tiles
 constexpr int RF_WORDS = 128;    // ints of Ctx::rf_bar (the refinement round kernel's barrier and error words,
                                  // the refinement's convergence gate)
