@@ -4,8 +4,7 @@
 // runs a batch of iterations per launch.
 //
 // One BiCGSTAB iteration is two GEMVs and three vector updates; as separate launches it is about
-// nine kernels.  This form serves the systems whose matrix does not fit on the SMs (N > 2048; smaller
-// ones: bicg_resident.cu).  Here the phases are
+// nine kernels.  This form serves N > 6144 (smaller systems: bicg_resident.cu).  Here the phases are
 // separated by a grid-wide barrier (sense counter in global memory, bounded wait), the scalars are
 // recomputed redundantly by every CTA from the same per-row-block partial sums (fixed order, so every
 // CTA holds the same bits), and the host polls the done flag once per batch of iterations.

@@ -1,9 +1,10 @@
-// BiCGSTAB with the matrix resident on the SMs (the reference's default solver, Simulation.cpp:49-53:
+// BiCGSTAB with the vectors resident on the SMs (the reference's default solver, Simulation.cpp:49-53:
 // Jacobi preconditioner, zero start, tolerance DBL_EPSILON on the recursive residual, at most 2N
-// iterations, shadow-residual restart): the whole solve in one cooperative launch, for systems whose
-// matrix fits the register files and shared memories of the GPU (N <= 2048: 33.6 MB).
+// iterations, shadow-residual restart): the whole solve in one cooperative launch, for N <= 6144.  Up to
+// N = 2048 (33.6 MB) the matrix too stays in the register files and shared memories of the GPU; above, it is
+// streamed from L2 and HBM.
 //
-// What bounds it: at these sizes a product reads nothing from outside the SM and takes well under a
+// What bounds it, matrix resident: a product reads nothing from outside the SM and takes well under a
 // microsecond, so an iteration costs its two all-to-all exchanges and the chain of dot products.
 //   * A CTA owns 16 rows (or N / SMs, if that is more), a thread up to 28 entries of one row in
 //     registers and the rest in shared memory.  Few CTAs: every CTA reads every published vector, and
@@ -22,7 +23,15 @@
 //     1.3 to 1.8 us per exchange over 50 to 140 CTAs; a counter barrier and a read of the vector take
 //     1.9 to 2.4 us.
 // Measured (B200, whole solve, against k_pbicg in batches of 64 iterations): N = 162: 0.10 ms (0.63),
-// N = 812 with the wall image: 0.23 ms (1.13), N = 1442: 0.35 ms (1.66), N = 1962: 0.59 ms.
+// N = 812 with the wall image: 0.23 ms (1.13), N = 1442: 0.35 ms (1.66), N = 1962: 0.54 ms.
+//
+// Matrix streamed: bound by the two reads of the matrix per iteration.  Each thread copies two rows of its
+// columns (16 bytes) into a ring of its own in shared memory, 12 copies ahead (98 KB in flight per SM, no
+// registers held, no barrier: a thread reads only what it copied), and the copies run on through the exchanges.
+// 64 MB of the matrix are marked to stay in L2 (evict_last, the rest evict_first).  Per iteration: N = 4002:
+// 38 us (6.7 TB/s of matrix reads) against 91 us for k_pbicg; 42 us without the marks, 47 us with 100 MB marked.
+// With loads into registers instead of the ring 48 us; with a TMA ring of row slabs 71 us (a slab's rows are
+// 224 bytes, too short for the copy engine).  N = 2562: 24 us; N = 5762: 84 us.
 //
 // A wait is bounded (Ctx::wait_limit): a warp that gives up sets the error word and its CTA returns; the
 // others then run out of their own waits.  The host finishes the solve with the multi-kernel form.
@@ -39,10 +48,14 @@ namespace {
 
 constexpr int RB_T = 512;
 constexpr int RB_WARPS = RB_T / 32;
+constexpr int RB_D8 = 12, RB_D12 = 8;  // streamed: copies in flight per thread, up to 4096 and 6144 unknowns
+constexpr int RB_SMEM = 226 * 1024;
 constexpr double RB_EPS = 2.220446049250313080847e-16;
 
 struct RBArgs {
-    int n, rows, nv, npart, maxit;  // rows per CTA; doubles of the input vector and of the row partials
+    int n, ld, rows, nv, npart, maxit;  // rows per CTA; doubles of the input vector and of the row partials
+    int nk;                            // streamed: columns per thread
+    float keep;                        // streamed: share of the matrix to keep in L2
     const double* A;
     const double* b;
     double* x;
@@ -52,8 +65,8 @@ struct RBArgs {
     long long wait_limit;      // bound of each exchange wait, SM clock cycles
 };
 
-// Two sums over the CTA's threads, the same bits in every thread and, from the same inputs, in every
-// CTA; false when some thread's exchange wait expired (!ok).  rs: 2 RB_WARPS doubles, written again only
+// Two sums over the CTA's threads, the same bits in every thread and, from the same inputs, in
+// every CTA; false when some thread's exchange wait expired (!ok).  rs: 2 RB_WARPS doubles, written again only
 // after another barrier of the CTA.
 __device__ __forceinline__ bool cta_sums(double* rs, double u, double w, bool ok, double& su, double& sw) {
 #pragma unroll
@@ -114,28 +127,64 @@ __device__ __forceinline__ bool collect(const ulonglong2* slots, int n, unsigned
     return true;
 }
 
+// 16 bytes (two rows of a column) into the thread's own ring slot, through L2 only; `in` false: zeros.
+__device__ __forceinline__ void ring_copy(double2* slot, const double* src, bool in, uint64_t pol) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(slot)),
+                 "l"(src), "r"(in ? 16 : 0), "l"(pol)
+                 : "memory");
+}
+
 enum { PH_V, PH_T, PH_RX, PH_RT };
 
-template <int K, int M>
+// D > 0: the matrix is streamed, D copies in flight per thread; D = 0: it is resident, M entries per thread in
+// registers and the rest in shared memory.
+template <int K, int M, int D>
 __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
-    extern __shared__ double smem[];
+    constexpr bool ST = D > 0;
+    extern __shared__ __align__(16) double smem[];
     const int n = a.n, np = (n + 1) & ~1, nv = a.nv, tid = threadIdx.x, rows = a.rows;
-    const int row0 = blockIdx.x * rows, nr = min(rows, n - row0), cstep = RB_T / rows;
-    double *vec = smem, *r0 = smem + nv, *invd = r0 + np, *part = invd + np, *red = part + a.npart;
+    const int row0 = blockIdx.x * rows, nr = min(rows, n - row0);
+    const int per = ST ? rows / 2 : rows, cstep = RB_T / per;  // threads down a column, columns side by side
+    // streamed: the ring; the input vector, shadow residual and Jacobi diagonal; row partials; sums; the slab
+    double2* ring = reinterpret_cast<double2*>(smem) + tid;  // slot d at d RB_T
+    double* vec = smem + (size_t)2 * D * RB_T;
+    double *r0 = vec + nv, *invd = r0 + np, *part = invd + np, *red = part + a.npart;
     double* slab = red + 6 * RB_WARPS;
-    const int i = tid % rows, c = tid / rows;  // the thread's row of the CTA and first column
+    const int i = tid % per * (ST ? 2 : 1), c = tid / per;  // the thread's (first) row of the CTA, first column
     const bool active = c < cstep && i < nr;
-    // the thread's entries of the own rows: columns c + q cstep, the first M in registers, the others
+    // the stream of a thread: its two rows of columns c, c + cstep, ..., product after product
+    uint64_t pol = 0;
+    const double* next = a.A + (size_t)min(c, n - 1) * a.ld + row0 + min(i, nr - 1);
+    int nextj = c, slot = 0;
+    auto advance = [&](int d) {
+        if (active) {
+            ring_copy(ring + d * RB_T, next, nextj < n, pol);
+            nextj += cstep;
+            next += (size_t)cstep * a.ld;
+            if (nextj >= a.nk * cstep) {  // the next product
+                nextj -= a.nk * cstep;
+                next -= (size_t)a.nk * cstep * a.ld;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (ST) {
+        asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(pol) : "f"(a.keep));
+#pragma unroll
+        for (int d = 0; d < D; ++d) advance(d);
+    }
+    // the thread's entries of the own rows (not ST): columns c + q cstep, the first M in registers, the others
     // (columns from M cstep on) in shared memory
-    double m[M];
+    double m[M ? M : 1];
 #pragma unroll
     for (int q = 0; q < M; ++q) {
         const int j = c + q * cstep;
-        m[q] = active && j < n ? __ldg(a.A + (size_t)j * n + row0 + i) : 0.0;
+        m[q] = active && j < n ? __ldg(a.A + (size_t)j * a.ld + row0 + i) : 0.0;
     }
-    if (active)
+    if (!ST && active)
         for (int j = c + M * cstep; j < n; j += cstep)
-            slab[(j - M * cstep) * rows + i] = __ldg(a.A + (size_t)j * n + row0 + i);
+            slab[(j - M * cstep) * rows + i] = __ldg(a.A + (size_t)j * a.ld + row0 + i);
     for (int e = n + tid; e < nv; e += RB_T) vec[e] = 0.0;  // read with the zero entries past column n
     // r (s between the two products), p (p - w v after the second), v of the thread's elements
     double r[K], p[K], v[K];
@@ -145,7 +194,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
         const int e = tid + k * RB_T;
         r[k] = p[k] = v[k] = 0.0;
         if (e < n) {
-            const double d = __ldg(a.A + (size_t)e * n + e), be = __ldg(a.b + e);
+            const double d = __ldg(a.A + (size_t)e * a.ld + e), be = __ldg(a.b + e);
             invd[e] = d != 0.0 ? 1.0 / d : 1.0;
             r0[e] = be;
             r[k] = be;
@@ -187,7 +236,22 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
             __syncthreads();
             // the own rows of A vec
             double acc[4] = {0.0, 0.0, 0.0, 0.0};
-            if (active) {
+            if (ST) {
+                const double* vc = vec + c;
+                for (int k = 0; k < a.nk; ++k) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(ST ? D - 1 : 0) : "memory");
+                    const double2 v = ring[slot * RB_T];
+                    const double xv = vc[k * cstep];
+                    acc[0] = fma(v.x, xv, acc[0]);
+                    acc[1] = fma(v.y, xv, acc[1]);
+                    advance(slot);
+                    slot = slot + 1 == D ? 0 : slot + 1;
+                }
+                if (active) {
+                    part[i * (cstep + 1) + c] = acc[0];
+                    part[(i + 1) * (cstep + 1) + c] = acc[1];
+                }
+            } else if (active) {
                 const double* vc = vec + c;
 #pragma unroll
                 for (int q = 0; q < M; ++q) acc[q & 3] = fma(m[q], vc[q * cstep], acc[q & 3]);
@@ -199,8 +263,8 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
                     for (int q = 0; q < 4; ++q) acc[q] = fma(sl[q * sst], vec[j + q * cstep], acc[q]);
                 }
                 for (; j < n; j += cstep, sl += sst) acc[0] = fma(sl[0], vec[j], acc[0]);
-                part[i * (cstep + 1) + c] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
             }
+            if (!ST && active) part[i * (cstep + 1) + c] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
             __syncthreads();
             const int lane = tid & 31;
             for (int q = tid >> 5; q < nr; q += RB_WARPS) {
@@ -221,7 +285,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
                 v[k] = t[k];
                 if (tid + k * RB_T < n) s0 += r0[tid + k * RB_T] * v[k];
             }
-            if (!cta_sums(red, s0, 0.0, ok, r0v, dummy)) return;
+            if (!cta_sums(red, s0, 0.0, ok, r0v, dummy)) break;
             alpha = rho / r0v;
             // s = r - alpha v; z = invd s
 #pragma unroll
@@ -239,7 +303,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
                 s0 += t[k] * t[k];
                 s1 += t[k] * r[k];
             }
-            if (!cta_sums(red + 2 * RB_WARPS, s0, s1, ok, tt, ts)) return;
+            if (!cta_sums(red + 2 * RB_WARPS, s0, s1, ok, tt, ts)) break;
             w = tt > 0.0 ? ts / tt : 0.0;
             bfac = (alpha / w) / rho;
             x += alpha * y + w * z;
@@ -258,7 +322,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
 #pragma unroll
             for (int k = 0; k < K; ++k)
                 if (tid + k * RB_T < n) vec[tid + k * RB_T] = t[k];
-            if (__syncthreads_or(!ok)) return;
+            if (__syncthreads_or(!ok)) break;
             phase = PH_RT;
         } else {  // r = b - A x, r0 = r
             double s0 = 0.0;
@@ -271,12 +335,13 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
                     s0 += r[k] * r[k];
                 }
             }
-            if (!cta_sums(red, s0, 0.0, ok, rho, dummy)) return;
+            if (!cta_sums(red, s0, 0.0, ok, rho, dummy)) break;
             r0_sq = rho;
             if (restarts++ == 0) iters = 0;
             phase = PH_V;
         }
     }
+    if (ST) asm volatile("cp.async.wait_all;" ::: "memory");
     if (tid < nr) a.x[row0 + tid] = x;
     if (blockIdx.x == 0 && tid == 0) {
         a.sc->rhs_sq = bb;
@@ -287,16 +352,16 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
     }
 }
 
-template <int K, int M>
+template <int K, int M, int D>
 cudaError_t rb_launch(const RBArgs& a, int grid, size_t smem, cudaStream_t s) {
     static std::atomic<uint64_t> ready{0};
     if (!once_per_device(ready, [] {
-            return cudaFuncSetAttribute(k_bicg_resident<K, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
-                   cudaSuccess;
+            return cudaFuncSetAttribute(k_bicg_resident<K, M, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        RB_SMEM) == cudaSuccess;
         }))
         return cudaErrorUnknown;
     void* args[] = {const_cast<RBArgs*>(&a)};
-    return cudaLaunchCooperativeKernel((void*)k_bicg_resident<K, M>, grid, RB_T, args, smem, s);
+    return cudaLaunchCooperativeKernel((void*)k_bicg_resident<K, M, D>, grid, RB_T, args, smem, s);
 }
 
 }  // namespace
@@ -312,29 +377,56 @@ int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaS
     if (!coop || n > RB_MAX_N || maxit > 4 * RB_MAX_N) return BEM_ERR_STATE;
     RBArgs a{};
     a.n = n;
-    a.rows = std::max(std::min(n, 16), (n + sms - 1) / sms);
-    const int grid = (n + a.rows - 1) / a.rows, np = (n + 1) & ~1, cstep = RB_T / a.rows;
-    const int K = (n + RB_T - 1) / RB_T;
-    const int M = K == 1 ? (n <= 8 * cstep ? 8 : 16) : K == 2 ? 28 : K == 3 ? 24 : 20;
-    a.nv = std::max(np, M * cstep);
-    a.nv += a.nv & 1;
-    a.npart = a.rows * (cstep + 1);
-    const size_t smem = sizeof(double) * (a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS +
-                                          (size_t)std::max(0, n - M * cstep) * a.rows);
-    if (smem > 227 * 1024) return BEM_ERR_STATE;
+    a.ld = n;
     a.maxit = maxit;
-    a.A = A;
     a.b = b;
     a.x = x;
     a.ex = reinterpret_cast<ulonglong2*>(c.rbicg);
-    a.seq = ++c.rbicg_solves << 32;
     a.sc = c.sc;
     a.wait_limit = c.wait_limit;
+    const bool stream = n > RB_RES_N;
+    const int np = (n + 1) & ~1, K = (n + RB_T - 1) / RB_T;
+    int grid = 0;
+    size_t smem = 0;
+    if (stream) {
+        a.rows = ((n + sms - 1) / sms + 1) & ~1;  // even: a copy takes two rows
+        grid = (n + a.rows - 1) / a.rows;
+        const int cstep = RB_T / (a.rows / 2), D = K <= 8 ? RB_D8 : RB_D12;
+        a.nk = (n + cstep - 1) / cstep;
+        a.nv = (a.nk * cstep + 1) & ~1;
+        a.npart = a.rows * (cstep + 1);
+        smem = sizeof(double) * ((size_t)2 * D * RB_T + a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS);
+        if (smem > RB_SMEM || a.rows > 2 * RB_T || a.nk < D || !c.LU) return BEM_ERR_STATE;
+        // the part of the matrix that the L2 can hold beside the stream
+        a.keep = (float)std::min(1.0, RB_KEEP / (8.0 * n * n));
+        if (n % 2 || reinterpret_cast<uintptr_t>(A) % 16) {  // copies of 16 bytes: a matrix with an even stride
+            a.ld = (n + 1) & ~1;
+            BEM_CUDA(c, cudaMemcpy2DAsync(c.LU, sizeof(double) * a.ld, A, sizeof(double) * n, sizeof(double) * n, n,
+                                          cudaMemcpyDeviceToDevice, s));
+            A = c.LU;
+        }
+    } else {
+        a.rows = std::max(std::min(n, 16), (n + sms - 1) / sms);
+        grid = (n + a.rows - 1) / a.rows;
+        const int cstep = RB_T / a.rows;
+        const int M = K == 1 ? (n <= 8 * cstep ? 8 : 16) : K == 2 ? 28 : K == 3 ? 24 : 20;
+        a.nv = std::max(np, M * cstep);
+        a.nv += a.nv & 1;
+        a.npart = a.rows * (cstep + 1);
+        smem = sizeof(double) *
+               (a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS + (size_t)std::max(0, n - M * cstep) * a.rows);
+        if (smem > RB_SMEM) return BEM_ERR_STATE;
+    }
+    a.A = A;
+    a.seq = ++c.rbicg_solves << 32;
     KLAUNCH();
-    const cudaError_t e = K == 1   ? (M == 8 ? rb_launch<1, 8>(a, grid, smem, s) : rb_launch<1, 16>(a, grid, smem, s))
-                          : K == 2 ? rb_launch<2, 28>(a, grid, smem, s)
-                          : K == 3 ? rb_launch<3, 24>(a, grid, smem, s)
-                                   : rb_launch<4, 20>(a, grid, smem, s);
+    const cudaError_t e = stream   ? (K <= 8 ? rb_launch<8, 0, RB_D8>(a, grid, smem, s)
+                                             : rb_launch<12, 0, RB_D12>(a, grid, smem, s))
+                          : K == 1 ? (n <= 8 * (RB_T / a.rows) ? rb_launch<1, 8, 0>(a, grid, smem, s)
+                                                               : rb_launch<1, 16, 0>(a, grid, smem, s))
+                          : K == 2 ? rb_launch<2, 28, 0>(a, grid, smem, s)
+                          : K == 3 ? rb_launch<3, 24, 0>(a, grid, smem, s)
+                                   : rb_launch<4, 20, 0>(a, grid, smem, s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return BEM_ERR_CUDA;

@@ -1,8 +1,9 @@
-"""The resident BiCGSTAB (one cooperative launch, matrix on the SMs) at the edges of its size classes.
+"""The resident BiCGSTAB (one cooperative launch) at the edges of its size classes.
 
 solve_system takes any dense matrix, so the sizes are picked freely: fewer rows than a CTA holds, one more
-than a multiple of the rows per CTA, the steps of the elements per thread (512, 1024, 1536, 2048) and of the
-entries kept in registers (columns beyond them sit in shared memory).  BiCGSTAB stops at a recursive
+than a multiple of the rows per CTA, the steps of the elements per thread (512, 1024, 1536, 2048, 4096, 6144) and of
+the entries kept in registers (columns beyond them sit in shared memory); above 2048 the matrix is streamed
+(odd sizes from a copy with an even stride), above 6144 the older persistent form takes over.  BiCGSTAB stops at a recursive
 residual of DBL_EPSILON; with a matrix of condition about 2 the solution is then within a few hundred
 roundings of LAPACK's (tolerance 1e-12).
 """
@@ -42,7 +43,7 @@ def system(n, seed):
     return np.asfortranarray(np.eye(n) + 0.3 * r.standard_normal((n, n)) / np.sqrt(n)), r.standard_normal(n)
 
 
-@pytest.mark.parametrize("n", [5, 15, 16, 17, 257, 512, 513, 897, 1024, 1025, 1536, 1537, 2047, 2048, 2049])
+@pytest.mark.parametrize("n", [5, 15, 16, 17, 257, 512, 513, 897, 1024, 1025, 1536, 1537, 2047, 2048, 2049, 2050, 3333, 4096, 4097, 6143, 6144, 6145])
 def test_matches_lapack_at_size_edges(n):
     v, f = uv_sphere(n)
     assert len(v) == n
@@ -58,7 +59,7 @@ def test_matches_lapack_at_size_edges(n):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [42, 700])
+@pytest.mark.parametrize("n", [42, 700, 2345])
 def test_iterates_match_the_multikernel_form(n):
     # the first iterates, cut off by max_iters, are those of the separate kernels up to rounding (the
     # recurrence amplifies it little in three iterations: 1e-12)
