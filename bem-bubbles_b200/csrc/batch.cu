@@ -99,9 +99,6 @@ __global__ void __launch_bounds__(BG_ROWS) k_bgemv(const int4* __restrict__ item
     if (threadIdx.x == 0) cnt[B.rbase + rb] = 0u;
 }
 
-// Per-block statistics (BSTAT_W doubles per block)
-enum { BS_BB = 0, BS_FIRST = 1, BS_LAST = 2, BS_RHO = 3, BS_STEPS = 4, BS_CONV = 5, BSTAT_W = 8 };
-
 // Start of a solve: ||b_b||^2, statistics reset; a zero right-hand side gives x_b = 0, converged.
 __global__ void __launch_bounds__(BG_ROWS) k_binit(const BlockInfo* __restrict__ blk, const double* __restrict__ b,
                                                    double* __restrict__ x, double* __restrict__ st,
@@ -158,6 +155,10 @@ constexpr int BATCH_KMAX = 8;
 int batch_mixed_solve(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s) {
     const double tol = c.prm.mixed_tol > 0 ? c.prm.mixed_tol : 1e-12;
     const int nb = c.nblk;
+    if (c.bteam && refine_batch(c, A, b, x, BATCH_KMAX, tol, c.bstat + (size_t)BSTAT_W * nb, s) == BEM_OK) {
+        c.stats.solves++;
+        return BEM_OK;
+    }
     double* rn = c.brnorm;
     KLAUNCH(), k_binit<<<nb, BG_ROWS, 0, s>>>(c.blk, b, x, c.bstat, c.bconv);
     const int dgrid = (nb * 32 + 255) / 256;
@@ -211,10 +212,11 @@ int batch_setup_solver(Ctx& c) {
     if ((rc = upload_vec(c, &c.gv_items, items)) || (rc = upload_vec(c, &c.blk, c.h_blk)) ||
         (rc = dalloc(c, &c.bpart, (size_t)pofs)) || (rc = dalloc(c, &c.bcnt, (size_t)rbase)) ||
         (rc = dalloc(c, &c.brnorm, (size_t)rbase)) || (rc = dalloc(c, &c.bconv, (size_t)c.nblk)) ||
-        (rc = dalloc(c, &c.bstat, (size_t)BSTAT_W * c.nblk)))
+        (rc = dalloc(c, &c.bstat, (size_t)BSTAT_W * c.nblk + 1)))
         return rc;
     BEM_CUDA(c, cudaMemset(c.bcnt, 0, sizeof(unsigned) * (size_t)rbase));
-    BEM_CUDA(c, cudaMallocHost((void**)&c.bstat_h, sizeof(double) * BSTAT_W * (size_t)c.nblk));  // freed by free_all
+    BEM_CUDA(c, cudaMemset(c.bstat, 0, sizeof(double) * (BSTAT_W * (size_t)c.nblk + 1)));
+    BEM_CUDA(c, cudaMallocHost((void**)&c.bstat_h, sizeof(double) * (BSTAT_W * (size_t)c.nblk + 1)));  // freed by free_all
     c.bmax_n = 0;
     for (auto& B : c.h_blk) c.bmax_n = std::max(c.bmax_n, B.n);
     const size_t mx = (size_t)c.bmax_n * c.bmax_n, np = (size_t)tc_pad(c.bmax_n) * tc_pad(c.bmax_n);
@@ -225,7 +227,7 @@ int batch_setup_solver(Ctx& c) {
     c.tcp = planes;
     BEM_CUDA(c, cudaMemset(c.tc_err, 0, sizeof(int)));
     c.bvalid.assign((size_t)c.nblk, 0);
-    return BEM_OK;
+    return refine_batch_setup(c);
 }
 
 // Newton-Schulz refresh of block b's approximate inverse against its current G block: one step
@@ -240,7 +242,7 @@ static int refresh_block(Ctx& c, const double* A, int b, cudaStream_t s) {
         if (rc) return rc;
         if (e < 0.9) {
             c.stats.precond_refresh++;
-            return BEM_OK;
+            return refine_batch_inverse(c, b, s);
         }
     }
     c.bvalid[(size_t)b] = 0;
@@ -248,7 +250,7 @@ static int refresh_block(Ctx& c, const double* A, int b, cudaStream_t s) {
     if (rc) return rc;
     c.bvalid[(size_t)b] = 1;
     c.stats.precond_refresh++;
-    return BEM_OK;
+    return refine_batch_inverse(c, b, s);
 }
 
 // Approximate inverses of every block that has none, from the G blocks currently assembled.
@@ -266,8 +268,21 @@ int batch_build_inverses(Ctx& c, cudaStream_t s) {
 // a block missed the tolerance within the refinement steps (the caller re-runs the step).
 int batch_after_step(Ctx& c, cudaStream_t s, bool* redo) {
     *redo = false;
-    BEM_CUDA(c, cudaMemcpyAsync(c.bstat_h, c.bstat, sizeof(double) * BSTAT_W * (size_t)c.nblk, cudaMemcpyDeviceToHost, s));
+    double* expired = c.bstat + (size_t)BSTAT_W * c.nblk;
+    BEM_CUDA(c, cudaMemcpyAsync(c.bstat_h, c.bstat, sizeof(double) * (BSTAT_W * (size_t)c.nblk + 1), cudaMemcpyDeviceToHost,
+                                s));
     BEM_CUDA(c, cudaStreamSynchronize(s));
+    if (c.bstat_h[(size_t)BSTAT_W * c.nblk] != 0.0) {
+        // an exchange wait of the resident refinement ran out: the step starts over with the separate launches,
+        // which the context keeps (and the graph, captured with the other, goes)
+        c.stats.wait_expired++;
+        c.bteam = 0;
+        if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
+        c.graph_exec = nullptr;
+        BEM_CUDA(c, cudaMemsetAsync(expired, 0, sizeof(double), s));
+        *redo = true;
+        return BEM_OK;
+    }
     double worst = 0.0;
     for (int b = 0; b < c.nblk; ++b) {
         const double* q = c.bstat_h + (size_t)BSTAT_W * b;

@@ -52,7 +52,7 @@ static void free_all(Ctx& c, bool keep_blocks = false) {
     c.pbicg = nullptr;
     c.rbicg = nullptr;
     c.lu_aux = nullptr;
-    c.Xinv = c.Tw = c.G32 = nullptr;
+    c.Xinv = c.Xpad = c.Tw = c.G32 = nullptr;
     c.tcp = nullptr;
     c.tc_err = nullptr;
     c.V = c.Z = nullptr;
@@ -75,6 +75,12 @@ static void free_all(Ctx& c, bool keep_blocks = false) {
     c.brnorm = nullptr;
     c.bconv = nullptr;
     c.bstat = nullptr;
+    c.bteam = 0;
+    c.blist = c.boff = nullptr;
+    c.bxoff = nullptr;
+    c.Xbpad = nullptr;
+    c.bslots = nullptr;
+    c.bnumber = nullptr;
     c.bvalid.clear();
     c.part_block.clear();
     c.h_ppar.clear();
@@ -622,6 +628,7 @@ static int alloc_mixed(Ctx& c) {
         (rc = dalloc(c, &planes, 4 * np)) || (rc = dalloc(c, &c.tc_err, 1)) ||
         (rc = dalloc(c, &c.V, n * (size_t)(c.gmres_m + 1))) || (rc = dalloc(c, &c.Z, n * (size_t)c.gmres_m)))
         return rc;
+    if (refine_resident_words(c.topo.N) && (rc = dalloc(c, &c.Xpad, refine_resident_words(c.topo.N)))) return rc;
     c.tcp = planes;
     BEM_CUDA(c, cudaMemset(c.tc_err, 0, sizeof(int)));
     return BEM_OK;
@@ -1065,7 +1072,7 @@ static int batch_steps(Ctx& c, double dt, int steps, bool graph) {
     for (int k = 0; k < steps; ++k) {
         BEM_CUDA(c, cudaMemcpyAsync(c.time_save, &c.sc->time, sizeof(double), cudaMemcpyDeviceToDevice, s));
         for (int attempt = 0;; ++attempt) {
-            if (graph) {
+            if (graph && c.graph_exec) {
                 BEM_CUDA(c, cudaGraphLaunch(c.graph_exec, s));
                 g_kernel_launches.fetch_add(c.graph_launches);
             } else if ((rc = rk4_step(c, dt, true, s))) {

@@ -93,6 +93,8 @@ struct Ctx {
     bool lu_rows_ok = true;    // the row-distributed panel is usable (cleared after a failed launch or wait)
     // mixed: approximate inverse (FP32), Krylov basis
     float* Xinv = nullptr;     // N*N column-major
+    float* Xpad = nullptr;     // X with its columns on 16 bytes, where N is not a multiple of four (small systems)
+    bool rfres_ok = true;      // the resident refinement is usable (cleared after a failed launch or wait)
     float* Tw = nullptr;       // N*N work for the Newton-Schulz refresh
     float* G32 = nullptr;      // N*N FP32 copy of G for the refresh GEMMs
     void* tcp = nullptr;       // 4 bf16 operand planes of the split-precision tensor-core GEMM
@@ -162,6 +164,15 @@ struct Ctx {
     double* bstat = nullptr;    // per block: BSTAT_W doubles (norms, contraction)
     double* bstat_h = nullptr;  // pinned host mirror
     std::vector<char> bvalid;   // per block: inverse built
+    // resident refinement of a batch (refine_resident.cu): CTAs per team (0: not planned), teams, their blocks,
+    // the inverses with padded strides, exchange slots, launch number
+    int bteam = 0, bteams = 0, bnv = 0, bnpart = 0;
+    int *blist = nullptr, *boff = nullptr;
+    long long* bxoff = nullptr;
+    std::vector<long long> h_bxoff;
+    float* Xbpad = nullptr;
+    double* bslots = nullptr;
+    unsigned long long* bnumber = nullptr;
     std::vector<int> part_block;      // block of each loose part
     std::vector<double> h_ppar;       // host mirror of ppar
     std::vector<int64_t> h_trigs, h_voff;  // the batch's triangles and block offsets (re-planning)

@@ -203,6 +203,19 @@ constexpr double RB_KEEP = 64e6;  // bytes of a streamed matrix kept in L2
 int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s);
 size_t rbicg_words(int64_t n);  // doubles of its exchange slots
 
+// refine_resident.cu: a round of the mixed solver's refinement as one launch (N <= RB_MAX_N)
+bool refine_resident_fits(const Ctx& c);
+int refine_resident(Ctx& c, const double* A, const double* b, double* x, const double* r, bool r_ready, int kmax,
+                    double tol, double slow, double* out, unsigned long long* number, cudaStream_t s);
+int refine_resident_inverse(Ctx& c, cudaStream_t s);  // after every change of c.Xinv
+size_t refine_resident_words(int64_t n);              // floats of c.Xpad
+// the same for a batch, all blocks in one launch
+int refine_batch_setup(Ctx& c);
+int refine_batch_inverse(Ctx& c, int b, cudaStream_t s);
+int refine_batch(Ctx& c, const double* A, const double* b, double* x, int kmax, double tol, double* err, cudaStream_t s);
+// Per-block statistics of a batched solve (BSTAT_W doubles per block, then one that an expired wait sets)
+enum { BS_BB = 0, BS_FIRST = 1, BS_LAST = 2, BS_RHO = 3, BS_STEPS = 4, BS_CONV = 5, BSTAT_W = 8 };
+
 // lu_panel.cu
 // The panel of another column-major n x n matrix (only its columns [k0, k0+nb) are touched); piv and
 // sing as c.piv and c.flag for c.LU.

@@ -1277,7 +1277,7 @@ static int refresh_inverse(Ctx& c, const double* A, cudaStream_t s, bool from_sc
         }
     }
     c.stats.precond_refresh++;
-    return BEM_OK;
+    return refine_resident_inverse(c, s);
 }
 
 int mixed_refresh(Ctx& c, const double* A, cudaStream_t s, bool from_scratch) {
@@ -1612,10 +1612,16 @@ int mixed_solve(Ctx& c, const double* A, const double* b, double* x, cudaStream_
     constexpr int KMAX = 12;
     double* pb = c.red;        // nrb
     double* pr = c.red + nrb;  // (KMAX+1)*nrb
-    if (r0_ready)
-        KLAUNCH(), k_rowblock_norm2x2<<<nrb, GV_ROWS, 0, s>>>(n, b, pb, c.r, pr);
-    else
-        KLAUNCH(), k_rowblock_norm2<<<nrb, GV_ROWS, 0, s>>>(n, b, pb);
+    // One launch per round with the convergence test inside, where the system is small enough; the flags ask
+    // for the separate launches or for their cooperative form
+    bool resident = !(c.prm.flags & (BEM_FLAG_REFINE_PERSISTENT | BEM_FLAG_NO_IR_GATE)) && refine_resident_fits(c);
+    auto norms = [&]() {  // |b|^2 and, when it is at hand, |r|^2 by row blocks, for the separate launches
+        if (r0_ready)
+            KLAUNCH(), k_rowblock_norm2x2<<<nrb, GV_ROWS, 0, s>>>(n, b, pb, c.r, pr);
+        else
+            KLAUNCH(), k_rowblock_norm2<<<nrb, GV_ROWS, 0, s>>>(n, b, pb);
+    };
+    if (!resident) norms();
     // The first round runs K steps and then up to IR_EXTRA more whose GEMVs are gated on the device:
     // a check after each residual from the K-th on stores the step at which the host's convergence
     // rule holds, and the gated GEMVs after it return at once.  A solve whose step count was guessed
@@ -1653,6 +1659,60 @@ int mixed_solve(Ctx& c, const double* A, const double* b, double* x, cudaStream_
         ++rounds;
         ++c.stats.ir_rounds;
         tail_valid = false;  // a round changes x
+        if (resident) {
+            unsigned long long number = 0;
+            if (refine_resident(c, A, b, x, c.r, round == 0 && r0_ready, KMAX, tol, 0.3, c.red, &number, s) != BEM_OK) {
+                resident = c.rfres_ok = false;
+                r0_ready = r0_ready && round == 0;
+                norms();
+                --round;
+                --rounds;
+                --c.stats.ir_rounds;
+                continue;
+            }
+            BEM_CUDA(c, cudaMemcpyAsync(host, c.red, sizeof(double) * (KMAX + 4), cudaMemcpyDeviceToHost, s));
+            if (round == 0 && tail) {
+                if (!c.solve_ev) BEM_CUDA(c, cudaEventCreateWithFlags(&c.solve_ev, cudaEventDisableTiming));
+                BEM_CUDA(c, cudaEventRecord(c.solve_ev, s));
+                const int trc = tail->run();
+                if (trc) return trc;
+                tail_valid = true;
+                BEM_CUDA(c, cudaEventSynchronize(c.solve_ev));
+            } else {
+                BEM_CUDA(c, cudaStreamSynchronize(s));
+            }
+            if (host[2] == (double)number) {
+                // an exchange wait ran out: x holds some rows of this round's update; any x is a valid iterate,
+                // so the separate launches go on from it
+                c.stats.wait_expired++;
+                resident = c.rfres_ok = false;
+                r0_ready = false;
+                tail_valid = false;
+                norms();
+                --round;
+                --rounds;
+                continue;
+            }
+            const int steps = (int)host[1];
+            c.stats.last_iters += steps;
+            if (host[0] == 0.0) {  // x = 0
+                tail_valid = false;
+                rel = 0.0;
+                converged = true;
+                break;
+            }
+            if (rel0 < 0) rel0 = host[3];
+            rel = host[3 + steps];
+            rho = 0.0;
+            for (int k = 0; k < steps; ++k)
+                if (host[3 + k] > 1e3 * tol) rho = std::max(rho, host[4 + k] / host[3 + k]);
+            if (rel <= tol) {
+                converged = true;
+                break;
+            }
+            if (!(rho < 0.3)) break;  // refinement too slow: GMRES below
+            continue;
+        }
         const bool skip_first = (round == 0 && r0_ready) || (round > 0 && r_fresh);
         const bool want = c.refine_ok && (c.prm.flags & BEM_FLAG_REFINE_PERSISTENT);
         const bool persistent = want && refine_round_persistent(c, A, b, x, pr, K, skip_first, s) == BEM_OK;
