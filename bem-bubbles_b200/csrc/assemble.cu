@@ -173,12 +173,11 @@ __global__ void k_triangle_records(int M, const double* __restrict__ x, const in
 // 1/sqrt(r2) for r2 > 0 in FP64: the hardware's approximate reciprocal square root
 // (rsqrt.approx.ftz.f64) refined by the binomial series of (1-d)^(-1/2) = 1 + d/2 + 3d^2/8 + ...
 // with d = 1 - r2*y0^2; truncation error 5d^3/16, far below the double rounding unit for the
-// estimate's relative error.
+// estimate's relative error.  The estimate has the upper 32 bits of a double only, so y0^2 is exact.
 __device__ __forceinline__ double rsqrt_fp64(double r2) {
     double y0;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(r2));
-    const double t = __dmul_rn(r2, y0);
-    const double d = fma(-t, y0, 1.0);
+    const double d = fma(-r2, __dmul_rn(y0, y0), 1.0);
     const double p = fma(0.375, d, 0.5);
     return fma(y0, __dmul_rn(d, p), y0);
 }
@@ -823,7 +822,7 @@ constexpr int COPY_WAIT_POLLS = 1 << 22;  // each poll may suspend the thread fo
 // A = |a - x|^2, B = |b - x|^2 - A = (a - x).2ab + |ab|^2 and C the same for ac, a point y with barycentric
 // weights (l0, l1, l2) lies at |y - x|^2 = A + l1 B + l2 C - W, W = l0 l1 |ab|^2 + l0 l2 |ac|^2 + l1 l2 |bc|^2,
 // so the points of an orbit (weights alpha, beta, beta in turn) share A + beta (B + C).  Layout: the three
-// vertex ids and the column slots (8 bits each) as four ints (0-1); a (2-4), 2ab (5-7), 2ac (8-10), |ab|^2,
+// vertices' columns as byte offsets into the tile's accumulators, three ints (0-1); a (2-4), 2ab (5-7), 2ac (8-10), |ab|^2,
 // |ac|^2 (11, 12), -area n (13-15), area (16), -W (17-23) and w phi (24-30) of the points.  The points are the
 // centroid, then the orbits' points by the vertex that has alpha.  Without the wall image 31-39 hold the
 // triangle's singular pairs: for row = vertex k of the triangle, the G entry of the column of vertex v at
@@ -864,7 +863,8 @@ __global__ void k_patch_records(int M, const double* __restrict__ x, const doubl
     const double ab2 = abx * abx + aby * aby + abz * abz, ac2 = acx * acx + acy * acy + acz * acz;
     const double bc2 = bcx * bcx + bcy * bcy + bcz * bcz;
     double* r = prec + (size_t)p * PREC;
-    *reinterpret_cast<int4*>(r) = make_int4(ia, ib, ic, pslot[p]);
+    const int sl = pslot[p], col = PATCH_ROWS * (int)sizeof(double);
+    *reinterpret_cast<int4*>(r) = make_int4((sl & 255) * col, (sl >> 8 & 255) * col, (sl >> 16 & 255) * col, 0);
     r[2] = ax;
     r[3] = ay;
     r[4] = az;
@@ -953,13 +953,17 @@ constexpr size_t patch_smem() {
 // One CTA per tile {patch, first row} of the work list, ROWS rows of the patch's block, one row per
 // thread.  G, the halo columns and the row partials are addressed through the patch's PatchInfo, so
 // the same kernel serves a single system (one block) and a batch of independent bubbles.
-// What bounds it: the pair loop, three quarters of it FP64 issue (N = 4002 without x0: 274 of 300 us, the FP64
-// pipe 66 % active; the finishing sums take 21 us, the column writes 4).  The records read as broadcasts keep
-// the shared-memory pipe at 64 % beside it, so fewer operations per pair gain less than their share: the
-// corner-distance form of the records (112 FP64 operations per pair against 123) took the kernel from 4.61 to
-// 4.44 ms at N = 16002 and from 318 to 309 us at N = 4002.  Measured slower at N = 4002: two rows per thread
-// with half the threads (a record read then serves two rows, 344 us), and a persistent form that defers tickets
-// and finishing sums by a tile (423 us); starting the SM's three CTAs apart changes nothing.
+// What bounds it: the pair loop, and there the register reads.  Measured (B200): an FP64 operation takes two issue
+// cycles of its SM quarter, three if it reads three different registers; beside one with two or three register
+// operands no other instruction issues for free, beside one with a single one (constants, repeated or just used
+// operands) some do.  So a pair's 112 FP64 operations and its other instructions add up, and more warps change
+// nothing (32 instead of 24 per SM with narrower patches: 4593 and 4602 us at N = 16002).  The shared-memory pipe
+// is 70 % busy beside it (records read as broadcasts).  Hence: no singular test in tiles without singular pairs,
+// column offsets ready in the record, two triangles per turn of the loop, y0^2 in rsqrt_fp64.  At N = 16002
+// 4.48 -> 4.10 ms, at N = 4002 311 -> 285 us, with the wall image at N = 1442 80 -> 74 us (four triangles per
+// turn: 4.19 ms).  Measured slower at N = 4002: two rows per thread with half the threads (a record read then
+// serves two rows, 299 us), and a persistent form that defers tickets and finishing sums by a tile (423 us before
+// these); starting the SM's three CTAs apart changes nothing.
 template <bool MIRROR, int ROWS, int MINB>
 __global__ void __launch_bounds__(ROWS, MINB)
     k_assemble_patch(const int2* __restrict__ work, const PatchInfo* __restrict__ pinfo,
@@ -973,7 +977,7 @@ __global__ void __launch_bounds__(ROWS, MINB)
     double* srec = psmem;                  // [PT_MAX][PREC], the patch's records
     double* acc = psmem + PT_MAX * PREC;   // [PCOLS][ROWS], this CTA's rows of the patch's columns
     __shared__ __align__(8) uint64_t bar;
-    __shared__ int s_pk[PCOLS], s_nc;
+    __shared__ int s_pk[PCOLS], s_v[PCOLS], s_nc, s_near;
     __shared__ double* s_dst[PCOLS];
     __shared__ double s_x0[PCOLS];
     const int tid = threadIdx.x;
@@ -990,7 +994,12 @@ __global__ void __launch_bounds__(ROWS, MINB)
         s_dst[tid] = h < 0 ? G + P.mbase + (long long)(v - P.vbase) * P.n : halo + h;  // where the column goes
         s_pk[tid] = patch_pk[p * PCOLS + tid];
         const unsigned used = __ballot_sync(0xffffffffu, v >= 0);  // the used slots come first
-        if (tid == 0) s_nc = __popc(used);
+        const unsigned near = __ballot_sync(0xffffffffu, v >= wk.y && v < wk.y + ROWS);
+        if (tid == 0) {
+            s_nc = __popc(used);
+            s_near = near != 0u;
+        }
+        s_v[tid] = v;
         s_x0[tid] = x0 && v >= 0 ? x0[v] : 0.0;
     }
 #pragma unroll 8
@@ -1014,31 +1023,43 @@ __global__ void __launch_bounds__(ROWS, MINB)
     }
     double hb = 0.0;  // the row's share of b over this patch's regular pairs
     const double wphi[3] = {__dmul_rn(c_pw[0], phii), __dmul_rn(c_pw[1], phii), __dmul_rn(c_pw[2], phii)};
-    double* mine = acc + tid;
-    for (int t = 0; t < (row ? P.nt : 0); ++t) {
-        const double* r = srec + t * PREC;
-        const int4 id = *reinterpret_cast<const int4*>(r);
-        double* a0 = mine + (id.w & 255) * ROWS;
-        double* a1 = mine + ((id.w >> 8) & 255) * ROWS;
-        double* a2 = mine + ((id.w >> 16) & 255) * ROWS;
-        if (i == id.x || i == id.y || i == id.z) {
-            // singular pair: without the wall image its G entries come with the records (the double
-            // layer of the flat own triangle vanishes); with it, k_singular_diag<true, true> adds both
-            if (!MIRROR) {
-                const double* sg = r + PR_SING + (i == id.x ? 0 : (i == id.y ? 3 : 6));
-                *a0 += sg[0];
-                *a1 += sg[1];
-                *a2 += sg[2];
+    // A tile with a vertex of the patch among its rows has singular pairs (without the wall image their G entries
+    // come with the records, and the double layer of the flat own triangle vanishes; with it,
+    // k_singular_diag<true, true> adds both); the other tiles run the loop without the test.
+    char* mine = reinterpret_cast<char*>(acc + tid);
+    const auto pairs = [&](auto near) {
+        int own = -1;  // the row's own column of the patch
+        if (decltype(near)::value)
+            for (int s = 0; s < s_nc; ++s)
+                if (s_v[s] == i) own = s * ROWS * (int)sizeof(double);
+#pragma unroll 2
+        for (int t = 0; t < (row ? P.nt : 0); ++t) {
+            const double* r = srec + t * PREC;
+            const int4 id = *reinterpret_cast<const int4*>(r);
+            double* a0 = reinterpret_cast<double*>(mine + id.x);
+            double* a1 = reinterpret_cast<double*>(mine + id.y);
+            double* a2 = reinterpret_cast<double*>(mine + id.z);
+            if (decltype(near)::value && (own == id.x || own == id.y || own == id.z)) {
+                if (!MIRROR) {
+                    const double* sg = r + PR_SING + (own == id.x ? 0 : (own == id.y ? 3 : 6));
+                    *a0 += sg[0];
+                    *a1 += sg[1];
+                    *a2 += sg[2];
+                }
+                continue;
             }
-            continue;
+            double g[3];
+            patch_pair<MIRROR>(r, xi0, xi1, xi2, wphi, g, hb);
+            const double area = r[16];
+            *a0 = fma(g[0], area, *a0);
+            *a1 = fma(g[1], area, *a1);
+            *a2 = fma(g[2], area, *a2);
         }
-        double g[3];
-        patch_pair<MIRROR>(r, xi0, xi1, xi2, wphi, g, hb);
-        const double area = r[16];
-        *a0 = fma(g[0], area, *a0);
-        *a1 = fma(g[1], area, *a1);
-        *a2 = fma(g[2], area, *a2);
-    }
+    };
+    if (s_near)
+        pairs(std::true_type{});
+    else
+        pairs(std::false_type{});
     const int il = i - P.vbase;
     if (row) {
         double gs = 0.0;
