@@ -12,9 +12,9 @@
 //                raw entries (the 4 pi rule makes row i depend on phi_j - phi_i)
 //   assembly     the derivative of every (row, triangle) integral with respect to the row's point
 //                and the triangle's vertices, contracted with those weights on the fly.
-// The assembly derivative runs as two passes that each recompute the pair terms: one thread per
-// triangle over a chunk of rows (per-triangle sums), one thread per row over a chunk of triangles
-// (per-row sums); partial sums are combined in a fixed order, so results are deterministic.
+// The assembly derivative runs as one pass over the pairs, one thread per triangle over a chunk of rows, with the
+// per-triangle sums in registers and the per-row sums in shared memory; partial sums are combined in a
+// fixed order, so results are deterministic.
 // Scope: free-space bubbles (no wall image), sigma = 0, device-evaluated field, single systems.
 #include <math.h>
 
@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "rsqrt.cuh"
 
 namespace bemb {
 
@@ -73,8 +74,8 @@ __device__ __forceinline__ void cross_vjp(v3 p, v3 q, v3 wb, v3& pb, v3& qb) {
 // ------------------------------------------------------------------------------------------------
 // Assembly derivative
 // ------------------------------------------------------------------------------------------------
-constexpr int AREC = 44;  // per-triangle record of the adjoint assembly
-// y_q (21), N = ab x bc (3), |N|, N.a, Psi_q (7), Phi_q (7), a (3), pad
+constexpr int AREC = 40;  // per-triangle record of the adjoint assembly, entry k of triangle t at k M + t:
+// y_q (21), N = ab x bc (3), |N|, N.a, |N| Psi_q (7), Phi_q (7)
 __global__ void k_adj_records(int M, const double* __restrict__ x, const int* __restrict__ tri,
                               const double* __restrict__ psi, const double* __restrict__ phi, double* __restrict__ rec) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -83,130 +84,141 @@ __global__ void k_adj_records(int M, const double* __restrict__ x, const int* __
     const v3 A = ld(x, ia), B = ld(x, ib), C = ld(x, ic);
     const v3 ab = B - A, bc = C - B;
     const v3 N = cr(ab, bc);
-    double* r = rec + (size_t)t * AREC;
+    const double nrm = sqrt(dt3(N, N));
+    const auto r = [&](int k) -> double& { return rec[(size_t)k * M + t]; };
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
         const double u = a_quv[q][0], v = a_quv[q][1];
-        r[3 * q] = (A.x + u * ab.x) + v * bc.x;
-        r[3 * q + 1] = (A.y + u * ab.y) + v * bc.y;
-        r[3 * q + 2] = (A.z + u * ab.z) + v * bc.z;
-        r[30 + q] = a_qc[q][0] * psi[ia] + a_qc[q][1] * psi[ib] + a_qc[q][2] * psi[ic];
-        r[37 + q] = a_qc[q][0] * phi[ia] + a_qc[q][1] * phi[ib] + a_qc[q][2] * phi[ic];
+        r(3 * q) = (A.x + u * ab.x) + v * bc.x;
+        r(3 * q + 1) = (A.y + u * ab.y) + v * bc.y;
+        r(3 * q + 2) = (A.z + u * ab.z) + v * bc.z;
+        r(26 + q) = nrm * (a_qc[q][0] * psi[ia] + a_qc[q][1] * psi[ib] + a_qc[q][2] * psi[ic]);
+        r(33 + q) = a_qc[q][0] * phi[ia] + a_qc[q][1] * phi[ib] + a_qc[q][2] * phi[ic];
     }
-    r[21] = N.x;
-    r[22] = N.y;
-    r[23] = N.z;
-    r[24] = sqrt(dt3(N, N));
-    r[25] = dt3(N, A);
-    r[26] = A.x;
-    r[27] = A.y;
-    r[28] = A.z;
-    r[29] = 0.0;
+    r(21) = N.x;
+    r(22) = N.y;
+    r(23) = N.z;
+    r(24) = nrm;
+    r(25) = dt3(N, A);
 }
 
-// One regular (row i, triangle t) pair, weights from mu_i, psi, phi:
+// Every regular (row i, triangle t) pair, weights from mu_i, psi, phi:
 //   J = |N| sum_q alpha_q / r_q - P sum_q eta_q / r_q^3,  P = N.(a - x_i),
-//   alpha_q = -mu_i Psi_q,  eta_q = mu_i (Phi_q - phi_i w_q).
-// Returns S1 = sum alpha/r, S3 = sum eta/r^3 and accumulates dJ/dz_q (z_q = y_q - x_i) into zb.
-__device__ __forceinline__ void pair_terms(const double* __restrict__ r, v3 xi, double mu, double phii, double& S1,
-                                           double& S3, v3* zb) {
-    const double nrm = r[24];
-    const double P = r[25] - (r[21] * xi.x + r[22] * xi.y + r[23] * xi.z);
-    S1 = 0.0;
-    S3 = 0.0;
+//   alpha_q = -mu_i Psi_q,  eta_q = mu_i (Phi_q - phi_i w_q);
+// with S1 = sum alpha / r, S3 = sum eta / r^3 and z_q = y_q - x_i.  Per triangle and row chunk (part_t): the sums of
+// |N| S1, S3, S3 x_i (3) and dJ/dz_q (21).  Per row and group of ADJ_T triangles (part_r): the sum of
+// S3 N - sum_q dJ/dz_q.
+//
+// What bounds it: the FP64 operations, about 200 per pair.  One thread per triangle with the record and the
+// triangle's sums in registers; the lanes of a warp take 32 different rows at a time, each row's sum waits for
+// them in the warp's own shared memory, so the pair terms are computed once for both sides.  At N = 1002: 39 us;
+// two passes that each formed the terms, with a square root and a division per point, took 141.
+constexpr int APART = 26, ADJ_T = 128, ADJ_R = 128;
+__global__ void __launch_bounds__(ADJ_T, 3)
+    k_adj_pairs(int M, int N, int rows, const double* __restrict__ rec, const int* __restrict__ tri,
+                const double* __restrict__ x, const double* __restrict__ mu, const double* __restrict__ phi,
+                double* __restrict__ part_t, double* __restrict__ part_r) {
+    __shared__ double srow[5][ADJ_R], sacc[ADJ_T / 32][3][ADJ_R];
+    const int t = blockIdx.x * ADJ_T + threadIdx.x, ch = blockIdx.y;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool have = t < M;
+    const int tt = have ? t : M - 1;
+    double r[AREC];
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-        const v3 z = {r[3 * q] - xi.x, r[3 * q + 1] - xi.y, r[3 * q + 2] - xi.z};
-        const double r2 = dt3(z, z);
-        const double inv = 1.0 / sqrt(r2);
-        const double inv3 = inv * inv * inv;
-        const double al = -mu * r[30 + q];
-        const double et = mu * (r[37 + q] - phii * a_w[q]);
-        S1 = fma(al, inv, S1);
-        S3 = fma(et, inv3, S3);
-        const double cf = -nrm * al * inv3 + 3.0 * P * et * inv3 * inv * inv;
-        zb[q] = zb[q] + cf * z;
-    }
-}
-
-// Triangle side: thread per triangle over rows [r0, r1); partial sums per (row chunk, triangle):
-// sum S1, sum S3, sum S3 x_i (3), dJ/dz_q (21).
-constexpr int APART = 26;
-__global__ void __launch_bounds__(128) k_adj_tri_pass(int M, int N, int rows_per_chunk, const double* __restrict__ rec,
-                                                       const int* __restrict__ tri, const double* __restrict__ x,
-                                                       const double* __restrict__ mu, const double* __restrict__ phi,
-                                                       double* __restrict__ part) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ch = blockIdx.y;
-    if (t >= M) return;
-    const int r0 = ch * rows_per_chunk, r1 = min(N, r0 + rows_per_chunk);
-    const int ia = tri[3 * t], ib = tri[3 * t + 1], ic = tri[3 * t + 2];
-    double rr[AREC];
-#pragma unroll
-    for (int k = 0; k < AREC; ++k) rr[k] = rec[(size_t)t * AREC + k];
+    for (int k = 0; k < AREC; ++k) r[k] = rec[(size_t)k * M + tt];
+    const int ia = tri[3 * tt], ib = tri[3 * tt + 1], ic = tri[3 * tt + 2];
+    const v3 Nv = {r[21], r[22], r[23]};
     v3 zb[7];
 #pragma unroll
     for (int q = 0; q < 7; ++q) zb[q] = {0.0, 0.0, 0.0};
     double s1 = 0.0, s3 = 0.0;
     v3 s3x = {0.0, 0.0, 0.0};
-    for (int i = r0; i < r1; ++i) {
-        if (i == ia || i == ib || i == ic) continue;  // singular pairs: k_adj_tri_final
-        const v3 xi = ld(x, i);
-        double S1, S3;
-        pair_terms(rr, xi, mu[i], phi[i], S1, S3, zb);
-        s1 += S1;
-        s3 += S3;
-        s3x = s3x + S3 * xi;
-    }
-    double* o = part + ((size_t)ch * M + t) * APART;
-    o[0] = s1;
-    o[1] = s3;
-    o[2] = s3x.x;
-    o[3] = s3x.y;
-    o[4] = s3x.z;
+    const int r1 = min(N, (ch + 1) * rows);
+    for (int r0 = ch * rows; r0 < r1; r0 += ADJ_R) {
+        const int nr = min(r1 - r0, ADJ_R);
+        for (int j = threadIdx.x; j < nr; j += ADJ_T) {
+            srow[0][j] = x[3 * (r0 + j)];
+            srow[1][j] = x[3 * (r0 + j) + 1];
+            srow[2][j] = x[3 * (r0 + j) + 2];
+            srow[3][j] = mu[r0 + j];
+            srow[4][j] = phi[r0 + j];
+        }
+        for (int j = lane; j < nr; j += 32) sacc[wid][0][j] = sacc[wid][1][j] = sacc[wid][2][j] = 0.0;
+        __syncthreads();
+        const int ja = ia - r0, jb = ib - r0, jc = ic - r0;
+        const int period = max(nr, 32);
+        for (int s = 0; s < period; ++s) {
+            const int e = s + lane, j = e < period ? e : e - period;
+            // singular pairs: k_adj_tri_final
+            if (have && j < nr && j != ja && j != jb && j != jc) {
+                const v3 xi = {srow[0][j], srow[1][j], srow[2][j]};
+                const double m = srow[3][j], ph = srow[4][j];
+                const double P3 = 3.0 * (r[25] - dt3(Nv, xi));
+                double S1 = 0.0, S3 = 0.0;
+                v3 zs = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-        o[5 + 3 * q] = zb[q].x;
-        o[6 + 3 * q] = zb[q].y;
-        o[7 + 3 * q] = zb[q].z;
+                for (int q = 0; q < 7; ++q) {
+                    const v3 z = {r[3 * q] - xi.x, r[3 * q + 1] - xi.y, r[3 * q + 2] - xi.z};
+                    const double inv = rsqrt_fp64(dt3(z, z));
+                    const double inv2 = inv * inv, inv3 = inv2 * inv;
+                    const double f = fma(-a_w[q], ph, r[33 + q]);
+                    S1 = fma(r[26 + q], inv, S1);
+                    S3 = fma(f, inv3, S3);
+                    const double cf = (m * inv3) * fma(P3, f * inv2, r[26 + q]);
+                    zb[q] = {fma(cf, z.x, zb[q].x), fma(cf, z.y, zb[q].y), fma(cf, z.z, zb[q].z)};
+                    zs = {fma(cf, z.x, zs.x), fma(cf, z.y, zs.y), fma(cf, z.z, zs.z)};
+                }
+                s1 = fma(-m, S1, s1);
+                S3 *= m;
+                s3 += S3;
+                s3x = {fma(S3, xi.x, s3x.x), fma(S3, xi.y, s3x.y), fma(S3, xi.z, s3x.z)};
+                sacc[wid][0][j] += fma(S3, Nv.x, -zs.x);
+                sacc[wid][1][j] += fma(S3, Nv.y, -zs.y);
+                sacc[wid][2][j] += fma(S3, Nv.z, -zs.z);
+            }
+            __syncwarp();  // the next lane takes the row
+        }
+        __syncthreads();
+        for (int j = threadIdx.x; j < nr; j += ADJ_T)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                part_r[((size_t)blockIdx.x * 3 + d) * N + r0 + j] =
+                    ((sacc[0][d][j] + sacc[1][d][j]) + sacc[2][d][j]) + sacc[3][d][j];
+        __syncthreads();
+    }
+    if (have) {
+        const auto o = [&](int k) -> double& { return part_t[((size_t)ch * APART + k) * M + t]; };
+        o(0) = s1;
+        o(1) = s3;
+        o(2) = s3x.x;
+        o(3) = s3x.y;
+        o(4) = s3x.z;
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            o(5 + 3 * q) = zb[q].x;
+            o(6 + 3 * q) = zb[q].y;
+            o(7 + 3 * q) = zb[q].z;
+        }
     }
 }
+static_assert(ADJ_T == 128, "the row sums of four warps");
 
-// Row side: thread per row over triangles [t0, t1); xbar_i partial per (triangle chunk, row).
-__global__ void __launch_bounds__(128) k_adj_row_pass(int N, int M, int tris_per_chunk, const double* __restrict__ rec,
-                                                       const int* __restrict__ tri, const double* __restrict__ x,
-                                                       const double* __restrict__ mu, const double* __restrict__ phi,
-                                                       double* __restrict__ part) {
+// The row side's partials and the triangle corners at each vertex: xbar_i += both.
+__global__ void k_adj_vert_final(int N, int ngroups, const double* __restrict__ part, const int* __restrict__ off,
+                                 const int* __restrict__ idx, const int* __restrict__ tri,
+                                 const double* __restrict__ tb, double* __restrict__ xbar) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ch = blockIdx.y;
     if (i >= N) return;
-    const int t0 = ch * tris_per_chunk, t1 = min(M, t0 + tris_per_chunk);
-    const v3 xi = ld(x, i);
-    const double m = mu[i], ph = phi[i];
-    v3 acc = {0.0, 0.0, 0.0};
-    for (int t = t0; t < t1; ++t) {
-        if (i == tri[3 * t] || i == tri[3 * t + 1] || i == tri[3 * t + 2]) continue;
-        const double* r = rec + (size_t)t * AREC;
-        v3 zb[7];
-#pragma unroll
-        for (int q = 0; q < 7; ++q) zb[q] = {0.0, 0.0, 0.0};
-        double S1, S3;
-        pair_terms(r, xi, m, ph, S1, S3, zb);
-        v3 zs = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int q = 0; q < 7; ++q) zs = zs + zb[q];
-        const v3 Nv = {r[21], r[22], r[23]};
-        acc = acc + (S3 * Nv - zs);
+    v3 s = {0.0, 0.0, 0.0}, c = {0.0, 0.0, 0.0};
+    for (int e = off[i]; e < off[i + 1]; ++e) {
+        const int t = idx[e];
+        const int k = tri[3 * t] == i ? 0 : (tri[3 * t + 1] == i ? 1 : 2);
+        c = c + ld(tb, 3 * t + k);
     }
-    put3(part, ch * N + i, acc);
-}
-
-__global__ void k_adj_row_final(int N, int nch, const double* __restrict__ part, double* __restrict__ xbar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    v3 s = {0.0, 0.0, 0.0};
-    for (int c = 0; c < nch; ++c) s = s + ld(part, c * N + i);
-    add3(xbar, i, s);
+#pragma unroll 4
+    for (int g = 0; g < ngroups; ++g)
+        s = s + v3{part[((size_t)g * 3) * N + i], part[((size_t)g * 3 + 1) * N + i], part[((size_t)g * 3 + 2) * N + i]};
+    add3(xbar, i, c + s);
 }
 
 // Singular pair VJP: collocation vertex P0 of its own triangle (P0, P1, P2) (rotated as in the
@@ -238,54 +250,76 @@ __device__ void singular_vjp(v3 P0, v3 P1, v3 P2, double wg0, double wg1, double
 }
 
 // Per triangle: the partial sums over row chunks in order, then the derivative with respect to its
-// vertices a, b, c; plus its three singular pairs.  Output tb[t] = (abar, bbar, cbar) (overwritten).
-__global__ void k_adj_tri_final(int M, int nch, const double* __restrict__ part, const double* __restrict__ rec,
-                                const int* __restrict__ tri, const double* __restrict__ x,
-                                const double* __restrict__ mu, const double* __restrict__ psi, double* __restrict__ tb) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= M) return;
-    double s[APART];
+// vertices a, b, c; plus its three singular pairs.  Output tb[t] = (abar, bbar, cbar) (overwritten).  A CTA takes 32
+// triangles: its warps share the sums' entries, then one warp the regular pairs and one each corner.
+constexpr int ATF_W = 8;
+__global__ void __launch_bounds__(32 * ATF_W)
+    k_adj_tri_final(int M, int nch, const double* __restrict__ part, const double* __restrict__ rec,
+                    const int* __restrict__ tri, const double* __restrict__ x, const double* __restrict__ mu,
+                    const double* __restrict__ psi, double* __restrict__ tb) {
+    __shared__ double ss[APART][32], so[4][9][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
+    const bool have = t < M;
+    const int tt = have ? t : M - 1;
+    constexpr int KW = (APART + ATF_W - 1) / ATF_W;
+    double sum[KW];
 #pragma unroll
-    for (int k = 0; k < APART; ++k) s[k] = 0.0;
+    for (int e = 0; e < KW; ++e) sum[e] = 0.0;
+#pragma unroll 4
     for (int c = 0; c < nch; ++c) {
-        const double* p = part + ((size_t)c * M + t) * APART;
+        const double* p = part + (size_t)c * APART * M + tt;
 #pragma unroll
-        for (int k = 0; k < APART; ++k) s[k] += p[k];
+        for (int e = 0; e < KW; ++e)
+            if (wid + e * ATF_W < APART) sum[e] += p[(size_t)(wid + e * ATF_W) * M];
     }
-    const double* r = rec + (size_t)t * AREC;
-    const int id[3] = {tri[3 * t], tri[3 * t + 1], tri[3 * t + 2]};
-    const v3 A = ld(x, id[0]), B = ld(x, id[1]), C = ld(x, id[2]);
-    const v3 ab = B - A, bc = C - B;
-    const v3 N = {r[21], r[22], r[23]};
-    const double nrm = r[24];
-    // Nbar = (sum S1) N/|N| - (sum S3) a + sum S3 x_i
-    const v3 Nb = ((s[0] / nrm) * N - s[1] * A) + v3{s[2], s[3], s[4]};
-    v3 Ab = -s[1] * N, Bb = {0.0, 0.0, 0.0}, Cb = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-        const double u = a_quv[q][0], v = a_quv[q][1];
-        const v3 z = {s[5 + 3 * q], s[6 + 3 * q], s[7 + 3 * q]};
-        Ab = Ab + (1.0 - u) * z;
-        Bb = Bb + (u - v) * z;
-        Cb = Cb + v * z;
-    }
-    v3 abb = {0.0, 0.0, 0.0}, bcb = {0.0, 0.0, 0.0};
-    cross_vjp(ab, bc, Nb, abb, bcb);
-    Ab = Ab - abb;
-    Bb = Bb + abb - bcb;
-    Cb = Cb + bcb;
-    // singular pairs: collocation vertex k, the triangle rotated to start there
-    v3 out[3] = {Ab, Bb, Cb};
-    const v3 P[3] = {A, B, C};
+    for (int e = 0; e < KW; ++e)
+        if (wid + e * ATF_W < APART) ss[wid + e * ATF_W][lane] = sum[e];
+    __syncthreads();
+    if (wid < 4) {
+        const int id[3] = {tri[3 * tt], tri[3 * tt + 1], tri[3 * tt + 2]};
+        v3 out[3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+        if (wid == 3) {
+            const v3 A = ld(x, id[0]), B = ld(x, id[1]), C = ld(x, id[2]);
+            const v3 ab = B - A, bc = C - B;
+            const v3 N = {rec[(size_t)21 * M + tt], rec[(size_t)22 * M + tt], rec[(size_t)23 * M + tt]};
+            const double nrm = rec[(size_t)24 * M + tt];
+            // Nbar = (sum S1) N/|N| - (sum S3) a + sum S3 x_i
+            const v3 Nb = ((ss[0][lane] / (nrm * nrm)) * N - ss[1][lane] * A) + v3{ss[2][lane], ss[3][lane], ss[4][lane]};
+            v3 Ab = -ss[1][lane] * N, Bb = {0.0, 0.0, 0.0}, Cb = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
-        const double m = mu[id[k]];
-        singular_vjp(P[k], P[k1], P[k2], -m * psi[id[k]], -m * psi[id[k1]], -m * psi[id[k2]], out[k], out[k1], out[k2]);
+            for (int q = 0; q < 7; ++q) {
+                const double u = a_quv[q][0], v = a_quv[q][1];
+                const v3 z = {ss[5 + 3 * q][lane], ss[6 + 3 * q][lane], ss[7 + 3 * q][lane]};
+                Ab = Ab + (1.0 - u) * z;
+                Bb = Bb + (u - v) * z;
+                Cb = Cb + v * z;
+            }
+            v3 abb = {0.0, 0.0, 0.0}, bcb = {0.0, 0.0, 0.0};
+            cross_vjp(ab, bc, Nb, abb, bcb);
+            out[0] = Ab - abb;
+            out[1] = Bb + abb - bcb;
+            out[2] = Cb + bcb;
+        } else {
+            // singular pair: collocation vertex k, the triangle rotated to start there (out in that order)
+            const int i0 = id[wid], i1 = id[(wid + 1) % 3], i2 = id[(wid + 2) % 3];
+            const double m = mu[i0];
+            singular_vjp(ld(x, i0), ld(x, i1), ld(x, i2), -m * psi[i0], -m * psi[i1], -m * psi[i2], out[0], out[1], out[2]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int v = wid == 3 ? k : (wid + k) % 3;  // the triangle's vertex
+            so[wid][3 * v][lane] = out[k].x;
+            so[wid][3 * v + 1][lane] = out[k].y;
+            so[wid][3 * v + 2][lane] = out[k].z;
+        }
     }
-    put3(tb, 3 * t, out[0]);
-    put3(tb, 3 * t + 1, out[1]);
-    put3(tb, 3 * t + 2, out[2]);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 9 * 32; e += 32 * ATF_W) {
+        const int k = e % 9, l = e / 9;  // tb in order
+        if (blockIdx.x * 32 + l < M)
+            tb[(size_t)blockIdx.x * 9 * 32 + e] = ((so[3][k][l] + so[0][k][l]) + so[1][k][l]) + so[2][k][l];
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -491,14 +525,22 @@ static int adj_alloc(Ctx& c, int steps) {
         (rc = dalloc(c, &w.ckt, (size_t)cap)))
         return rc;
     if (w.N != (int64_t)N) {
-        // row chunks of the triangle pass and triangle chunks of the row pass: about four CTAs per SM
-        // in each pass, at least 16 rows / triangles per chunk
+        // rows per CTA of the pair pass: of one to four waves of three CTAs per SM the fullest, 32 rows at least (a
+        // warp's lanes hold as many at a time)
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-        const int rch = std::max(1, std::min(nbk(4 * sms, nbk((int64_t)M, 128)), std::max(1, (int)N / 16)));
-        const int tch = std::max(1, std::min(nbk(4 * sms, nbk((int64_t)N, 128)), std::max(1, (int)M / 16)));
-        w.rch = rch;
-        w.tch = tch;
+        const int groups = nbk((int64_t)M, ADJ_T);
+        double fullest = 0.0;
+        for (int wave = 1; wave <= 4; ++wave) {
+            const int rows = std::max(32, nbk((int64_t)N, std::max(1, wave * 3 * sms / groups)));
+            const long long ctas = (long long)groups * nbk((int64_t)N, rows);
+            const double full = (double)ctas / ((double)nbk(ctas, 3 * sms) * 3 * sms);
+            if (full > 1.02 * fullest) {
+                fullest = full;
+                w.rows = rows;
+            }
+        }
+        const int rch = nbk((int64_t)N, w.rows);
         if ((rc = dalloc(c, &w.xs, 4 * 3 * N)) || (rc = dalloc(c, &w.ps, 4 * N)) || (rc = dalloc(c, &w.ks, 4 * 3 * N)) ||
             (rc = dalloc(c, &w.kps, 4 * N)) || (rc = dalloc(c, &w.psis, 4 * N)) || (rc = dalloc(c, &w.Gs, 4 * N * N)) ||
             (rc = dalloc(c, &w.Hs, 4 * N * N)) || (rc = dalloc(c, &w.kb, 4 * 3 * N)) || (rc = dalloc(c, &w.kpb, 4 * N)) ||
@@ -506,7 +548,7 @@ static int adj_alloc(Ctx& c, int steps) {
             (rc = dalloc(c, &w.psb, N)) || (rc = dalloc(c, &w.vb, 3 * N)) || (rc = dalloc(c, &w.wv, 6 * N)) ||
             (rc = dalloc(c, &w.psib, N)) || (rc = dalloc(c, &w.mu, N)) || (rc = dalloc(c, &w.r, N)) ||
             (rc = dalloc(c, &w.tb, 9 * M)) || (rc = dalloc(c, &w.tp, 3 * M)) || (rc = dalloc(c, &w.rec, AREC * M)) ||
-            (rc = dalloc(c, &w.partA, (size_t)rch * M * APART)) || (rc = dalloc(c, &w.partB, (size_t)tch * N * 3)) ||
+            (rc = dalloc(c, &w.partA, (size_t)rch * M * APART)) || (rc = dalloc(c, &w.partB, (size_t)groups * N * 3)) ||
             (rc = dalloc(c, &w.S, (size_t)c.topo.nparts + 1)) || (rc = dalloc(c, &w.red, (size_t)nbk(N, 8) * 16 + 64)) ||
             (rc = dalloc(c, &w.tsave, 2)) || (rc = dalloc(c, &w.iox, 3 * N)) || (rc = dalloc(c, &w.iop, N)))
             return rc;
@@ -607,12 +649,10 @@ static int adj_stage_reverse(Ctx& c, int st, cudaStream_t s) {
     KLAUNCH(), k_gemv_tcol<double><<<nbk(N, 8), 256, 0, s>>>(N, H, w.mu, w.psb, w.psb, 1.0, nullptr);
     // assembly derivative
     KLAUNCH(), k_adj_records<<<nbk(M, 128), 128, 0, s>>>(M, xs, T.tri, psi, ps, w.rec);
-    const int rpc = nbk(N, w.rch), tpc = nbk(M, w.tch);
-    KLAUNCH(), k_adj_tri_pass<<<dim3(nbk(M, 128), w.rch), 128, 0, s>>>(M, N, rpc, w.rec, T.tri, xs, w.mu, ps, w.partA);
-    KLAUNCH(), k_adj_tri_final<<<nbk(M, 128), 128, 0, s>>>(M, w.rch, w.partA, w.rec, T.tri, xs, w.mu, psi, w.tb);
-    KLAUNCH(), k_gather<<<nbk(N, 128), 128, 0, s>>>(N, T.csr_off, T.csr_idx, T.tri, w.tb, nullptr, w.xsb, nullptr);
-    KLAUNCH(), k_adj_row_pass<<<dim3(nbk(N, 128), w.tch), 128, 0, s>>>(N, M, tpc, w.rec, T.tri, xs, w.mu, ps, w.partB);
-    KLAUNCH(), k_adj_row_final<<<nbk(N, 128), 128, 0, s>>>(N, w.tch, w.partB, w.xsb);
+    const int nch = nbk(N, w.rows), groups = nbk(M, ADJ_T);
+    KLAUNCH(), k_adj_pairs<<<dim3(groups, nch), ADJ_T, 0, s>>>(M, N, w.rows, w.rec, T.tri, xs, w.mu, ps, w.partA, w.partB);
+    KLAUNCH(), k_adj_tri_final<<<nbk(M, 32), 32 * ATF_W, 0, s>>>(M, nch, w.partA, w.rec, T.tri, xs, w.mu, psi, w.tb);
+    KLAUNCH(), k_adj_vert_final<<<nbk(N, 128), 128, 0, s>>>(N, groups, w.partB, T.csr_off, T.csr_idx, T.tri, w.tb, w.xsb);
     return BEM_OK;
 }
 

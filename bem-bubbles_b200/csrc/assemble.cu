@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "ctx.h"
+#include "rsqrt.cuh"
 
 namespace bemb {
 
@@ -168,18 +169,6 @@ __global__ void k_triangle_records(int M, const double* __restrict__ x, const in
     // plane offset a.n: every quadrature point y_q satisfies y_q.n = a.n, so (y_q - x).n is one
     // number per (row, triangle) pair
     r[27] = ax * unx + ay * uny + az * unz;
-}
-
-// 1/sqrt(r2) for r2 > 0 in FP64: the hardware's approximate reciprocal square root
-// (rsqrt.approx.ftz.f64) refined by the binomial series of (1-d)^(-1/2) = 1 + d/2 + 3d^2/8 + ...
-// with d = 1 - r2*y0^2; truncation error 5d^3/16, far below the double rounding unit for the
-// estimate's relative error.  The estimate has the upper 32 bits of a double only, so y0^2 is exact.
-__device__ __forceinline__ double rsqrt_fp64(double r2) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(r2));
-    const double d = fma(-r2, __dmul_rn(y0, y0), 1.0);
-    const double p = fma(0.375, d, 0.5);
-    return fma(y0, __dmul_rn(d, p), y0);
 }
 
 // Orbit-form basis sums of the 7 kernel values k[0..6] (see c_orb): out_k = C + dA*kA_k + dB*kB_k.

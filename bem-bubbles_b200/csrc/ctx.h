@@ -14,7 +14,7 @@ namespace bemb {
 // step, adjoint vectors and the partial sums of the assembly derivative.
 struct AdjWork {
     int64_t N = 0;
-    int cap = 0, steps = 0, rch = 1, tch = 1;
+    int cap = 0, steps = 0, rows = 32;  // rows: of a CTA of the pair pass
     double dt = 0.0, bb = 0.0;
     double *ckx = nullptr, *ckp = nullptr, *ckt = nullptr;                  // checkpoints
     double *xs = nullptr, *ps = nullptr, *ks = nullptr, *kps = nullptr;     // 4 stages
