@@ -552,10 +552,44 @@ static int adj_alloc(Ctx& c, int steps) {
             (rc = dalloc(c, &w.S, (size_t)c.topo.nparts + 1)) || (rc = dalloc(c, &w.red, (size_t)nbk(N, 8) * 16 + 64)) ||
             (rc = dalloc(c, &w.tsave, 2)) || (rc = dalloc(c, &w.iox, 3 * N)) || (rc = dalloc(c, &w.iop, N)))
             return rc;
+        if (refine_resident_fits(c) && dalloc(c, &w.xt, N * ((N + 3) & ~(size_t)3)))
+            cudaGetLastError();  // no memory for it: the separate launches
     }
     w.N = (int64_t)N;
     w.cap = cap;
     return BEM_OK;
+}
+
+// mu = G^-T rhs in resident rounds (refine_resident.cu), as in mixed_solve; *done when the tolerance was met.
+static int solve_transposed_resident(Ctx& c, const double* G, const double* rhs, double* mu, double tol, bool* done,
+                                     cudaStream_t s) {
+    AdjWork& w = c.adj;
+    constexpr int K = 6;
+    double h[K + 4];
+    bool first = true;
+    for (int round = 0; round < 6; ++round) {
+        unsigned long long number = 0;
+        if (refine_resident_transposed(c, G, rhs, mu, first, w.xt, K, tol, w.red, &number, s) != BEM_OK) {
+            c.rfres_ok = false;
+            return BEM_OK;
+        }
+        BEM_CUDA(c, cudaMemcpyAsync(h, w.red, sizeof(h), cudaMemcpyDeviceToHost, s));
+        BEM_CUDA(c, cudaStreamSynchronize(s));
+        if (h[2] == (double)number) {  // an exchange wait ran out: the separate launches start over
+            c.stats.wait_expired++;
+            c.rfres_ok = false;
+            return BEM_OK;
+        }
+        first = false;
+        *done = h[0] == 0.0 || h[3 + (int)h[1]] <= tol;
+        if (*done) return BEM_OK;
+        if (round == 1 || round == 3) {  // slow: refresh the approximate inverse against this G
+            int rc = mixed_refresh(c, G, s, false);
+            if (rc) return rc;
+            first = true;
+        }
+    }
+    return c.fail(BEM_ERR_NOT_CONVERGED, "adjoint: transposed solve did not reach the tolerance");
 }
 
 // mu = G^-T rhs by refinement mu <- mu + X^T (rhs - G^T mu) from mu = 0; the residual in FP64, the
@@ -565,11 +599,16 @@ static int solve_transposed(Ctx& c, const double* G, const double* rhs, double* 
     const int n = (int)c.topo.N;
     const int nb = nbk(n, 8);
     const double tol = c.prm.mixed_tol > 0 ? c.prm.mixed_tol : 1e-12;
-    BEM_CUDA(c, cudaMemsetAsync(mu, 0, sizeof(double) * n, s));
     if (!c.xinv_valid) {  // forward solves by another solver: build the approximate inverse
         int rc = mixed_refresh(c, G, s, true);
         if (rc) return rc;
     }
+    if (w.xt && !(c.prm.flags & (BEM_FLAG_REFINE_PERSISTENT | BEM_FLAG_NO_IR_GATE)) && refine_resident_fits(c)) {
+        bool done = false;
+        int rc = solve_transposed_resident(c, G, rhs, mu, tol, &done, s);
+        if (rc || done) return rc;
+    }
+    BEM_CUDA(c, cudaMemsetAsync(mu, 0, sizeof(double) * n, s));
     constexpr int K = 6;
     std::vector<double> h((size_t)(K + 2) * nb);
     double rel = 1.0;

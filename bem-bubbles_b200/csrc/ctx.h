@@ -14,6 +14,7 @@ namespace bemb {
 // step, adjoint vectors and the partial sums of the assembly derivative.
 struct AdjWork {
     int64_t N = 0;
+    float* xt = nullptr;  // X^T of the resident transposed solve (small systems)
     int cap = 0, steps = 0, rows = 32;  // rows: of a CTA of the pair pass
     double dt = 0.0, bb = 0.0;
     double *ckx = nullptr, *ckp = nullptr, *ckt = nullptr;                  // checkpoints

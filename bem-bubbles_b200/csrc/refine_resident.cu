@@ -360,27 +360,49 @@ bool refine_resident_fits(const Ctx& c) {
     return c.rfres_ok && c.rbicg && c.LU && c.topo.N <= RB_MAX_N && (c.topo.N % 4 == 0 || c.Xpad);
 }
 
+// One launch over the system a (n, G, X and their strides, b, x, r set).
+static int rr_round(Ctx& c, RSys& a, const RRule& q, double* out, unsigned long long* number, cudaStream_t s) {
+    int sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.device);
+    if (!coop) return BEM_ERR_CUDA;
+    // 16 rows as in bicg_resident.cu, more where the SMs run out; a multiple of four (X's copies)
+    a.rows = std::max(16, ((a.n + sms - 1) / sms + 3) & ~3);
+    const int grid = (a.n + a.rows - 1) / a.rows;
+    int nv = 0, npart = 0;
+    rr_sizes(a.n, a.rows, &nv, &npart);
+    const size_t smem = rr_smem(nv, npart);
+    if (smem > RB_SMEM) return BEM_ERR_CUDA;
+    a.ex = reinterpret_cast<ulonglong2*>(c.rbicg);
+    a.ex_other = a.n;
+    *number = ++c.rbicg_solves;
+    a.seq = *number << 32;
+    double id = (double)*number;
+    void* args[] = {&a, (void*)&q, &nv, &npart, &out, &id};
+    KLAUNCH();
+    if (rr_launch_n(a.n, args, false, grid, smem, s) != cudaSuccess) {
+        cudaGetLastError();
+        return BEM_ERR_CUDA;
+    }
+    return BEM_OK;
+}
+
+// The share of G that the L2 holds beside X.
+static float rr_keep(int n) {
+    const double nn = (double)n * n;
+    return (float)std::max(0.0, std::min(1.0, (RB_KEEP - 4.0 * nn) / (8.0 * nn)));
+}
+
 // One round of at most kmax steps from x; out (3 + kmax + 1 doubles on the device, as k_refine_resident leaves
 // them); *number: the launch's.  BEM_ERR_CUDA: the launch failed, nothing done.
 int refine_resident(Ctx& c, const double* A, const double* b, double* x, const double* r, bool r_ready, int kmax,
                     double tol, double slow, double* out, unsigned long long* number, cudaStream_t s) {
     const int n = (int)c.topo.N;
-    int sms = 0, coop = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.device);
-    if (!coop) return BEM_ERR_CUDA;
     RSys a{};
     a.n = n;
     a.ldg = n;
     a.ldx = (n + 3) & ~3;
     a.X = c.Xpad ? c.Xpad : c.Xinv;
-    // 16 rows as in bicg_resident.cu, more where the SMs run out; a multiple of four (X's copies)
-    a.rows = std::max(16, ((n + sms - 1) / sms + 3) & ~3);
-    const int grid = (n + a.rows - 1) / a.rows;
-    int nv = 0, npart = 0;
-    rr_sizes(n, a.rows, &nv, &npart);
-    const size_t smem = rr_smem(nv, npart);
-    if (smem > RB_SMEM) return BEM_ERR_CUDA;
     if (n % 2 || reinterpret_cast<uintptr_t>(A) % 16) {  // copies of 16 bytes: a matrix with an even stride
         a.ldg = (n + 1) & ~1;
         BEM_CUDA(c, cudaMemcpy2DAsync(c.LU, sizeof(double) * a.ldg, A, sizeof(double) * n, sizeof(double) * n, n,
@@ -391,23 +413,55 @@ int refine_resident(Ctx& c, const double* A, const double* b, double* x, const d
     a.b = b;
     a.r = r_ready ? r : nullptr;
     a.x = x;
-    a.ex = reinterpret_cast<ulonglong2*>(c.rbicg);
-    a.ex_other = n;
-    *number = ++c.rbicg_solves;
-    a.seq = *number << 32;
     // a tenth of the tolerance, or one step past it: the last step is cheap, and a solve that only just meets
     // the tolerance would leave the solution less exact than the rounds of separate launches do
-    const double nn = (double)n * n;
-    RRule q{kmax, tol, tol >= 1e-13 ? 0.1 : 1.0, slow, c.wait_limit,
-            (float)std::max(0.0, std::min(1.0, (RB_KEEP - 4.0 * nn) / (8.0 * nn)))};
-    double id = (double)*number;
-    void* args[] = {&a, &q, &nv, &npart, &out, &id};
-    KLAUNCH();
-    if (rr_launch_n(n, args, false, grid, smem, s) != cudaSuccess) {
-        cudaGetLastError();
-        return BEM_ERR_CUDA;
+    const RRule q{kmax, tol, tol >= 1e-13 ? 0.1 : 1.0, slow, c.wait_limit, rr_keep(n)};
+    return rr_round(c, a, q, out, number, s);
+}
+
+// blockIdx.z = 0: G^T into gt (stride ldg); 1: X^T into xt (stride ldx).
+__global__ void __launch_bounds__(256)
+    k_transpose_gx(int n, const double* __restrict__ G, const float* __restrict__ X, double* __restrict__ gt, int ldg,
+                   float* __restrict__ xt, int ldx) {
+    __shared__ double tile[32][33];
+    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
+    const bool g = blockIdx.z == 0;
+    for (int k = ly; k < 32; k += 8)
+        if (r0 + lx < n && c0 + k < n) {
+            const size_t e = (size_t)(c0 + k) * n + r0 + lx;
+            tile[k][lx] = g ? G[e] : (double)X[e];
+        }
+    __syncthreads();
+    for (int k = ly; k < 32; k += 8)
+        if (c0 + lx < n && r0 + k < n) {
+            if (g)
+                gt[(size_t)(r0 + k) * ldg + c0 + lx] = tile[lx][k];
+            else
+                xt[(size_t)(r0 + k) * ldx + c0 + lx] = (float)tile[lx][k];
+        }
+}
+
+// The same round for G^T y = b through the transpose of the approximate inverse; xt: n columns of
+// (n + 3) & ~3 floats.  first: the transposes are made and y starts from zero.
+int refine_resident_transposed(Ctx& c, const double* G, const double* b, double* y, bool first, float* xt, int kmax,
+                               double tol, double* out, unsigned long long* number, cudaStream_t s) {
+    const int n = (int)c.topo.N, nt = (n + 31) / 32;
+    RSys a{};
+    a.n = n;
+    a.ldg = (n + 1) & ~1;
+    a.ldx = (n + 3) & ~3;
+    a.A = c.LU;
+    a.X = xt;
+    a.b = b;
+    a.r = first ? b : nullptr;
+    a.x = y;
+    if (first) {
+        KLAUNCH(), k_transpose_gx<<<dim3(nt, nt, 2), 256, 0, s>>>(n, G, c.Xinv, c.LU, a.ldg, xt, a.ldx);
+        BEM_CUDA(c, cudaMemsetAsync(y, 0, sizeof(double) * n, s));
     }
-    return BEM_OK;
+    // the separate launches always run six steps: two orders below the tolerance, or one step past it
+    const RRule q{kmax, tol, tol >= 1e-13 ? 0.01 : 1.0, INFINITY, c.wait_limit, rr_keep(n)};
+    return rr_round(c, a, q, out, number, s);
 }
 
 // The batch's plan: teams of CTAs and their blocks (longest first, each to the team with the least work), the
