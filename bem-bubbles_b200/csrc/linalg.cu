@@ -1074,13 +1074,18 @@ __global__ void k_ns_combine(int64_t nn, const float* __restrict__ X, const floa
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x)
         Xn[i] = 2.f * X[i] - P[i];
 }
-__global__ void k_eye_resid(int n, const float* __restrict__ T, double* __restrict__ part) {
+// ||I - T||_F^2 by CTA, a column at a time.  Bound by the read of T: at n = 4002 23 us; with 128 CTAs and a
+// division per entry it took 256.
+constexpr int EYE_CTAS = 4 * 148;
+__global__ void __launch_bounds__(256) k_eye_resid(int n, const float* __restrict__ T, double* __restrict__ part) {
     double s = 0.0;
-    const int64_t nn = (int64_t)n * n;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nn; e += (int64_t)gridDim.x * blockDim.x) {
-        int64_t j = e / n, i = e - j * n;
-        double d = (i == j ? 1.0 : 0.0) - (double)T[e];
-        s += d * d;
+    for (int j = blockIdx.x; j < n; j += gridDim.x) {
+        const float* col = T + (size_t)j * n;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < n; i += 256) {
+            const double d = (i == j ? 1.0 : 0.0) - (double)__ldg(col + i);
+            s = fma(d, d, s);
+        }
     }
     s = block_sum(s);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
@@ -1097,13 +1102,14 @@ int ns_step(Ctx& c, const NSJob& j, cudaStream_t s, double* eres, int terms) {
     const int64_t nn = (int64_t)n * n;
     int rc = tc_gemm(c, n, j.G32, j.X, j.T, c.tcp, c.tc_err, s, terms);  // T = G X
     if (rc) return rc;
-    KLAUNCH(), k_eye_resid<<<VBLK, VTHR, 0, s>>>(n, j.T, c.red);
-    KLAUNCH(), k_sum_partials<<<1, 32, 0, s>>>(c.red, VBLK, c.red + VBLK);
+    const int nc = std::min(n, EYE_CTAS);
+    KLAUNCH(), k_eye_resid<<<nc, 256, 0, s>>>(n, j.T, c.red);
+    KLAUNCH(), k_sum_partials<<<1, 32, 0, s>>>(c.red, nc, c.red + EYE_CTAS);
     if ((rc = tc_gemm(c, n, j.X, j.T, j.P, c.tcp, c.tc_err, s, terms))) return rc;  // P = X T
     KLAUNCH(), k_ns_combine<<<4 * 148, 256, 0, s>>>(nn, j.X, j.P, j.X);
     double v = 0.0;
     int herr = 0;
-    BEM_CUDA(c, cudaMemcpyAsync(&v, c.red + VBLK, sizeof(double), cudaMemcpyDeviceToHost, s));
+    BEM_CUDA(c, cudaMemcpyAsync(&v, c.red + EYE_CTAS, sizeof(double), cudaMemcpyDeviceToHost, s));
     BEM_CUDA(c, cudaMemcpyAsync(&herr, c.tc_err, sizeof(int), cudaMemcpyDeviceToHost, s));
     BEM_CUDA(c, cudaStreamSynchronize(s));
     if (herr) return c.fail(BEM_ERR_CUDA, "tensor-core GEMM: bounded wait expired (code " + std::to_string(herr) + ")");
