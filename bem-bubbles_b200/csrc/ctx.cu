@@ -118,14 +118,14 @@ struct HostTopo {
 };
 
 // Triangle patches of the G-only assembly, block by block (a single system is one block): recursive
-// coordinate bisection of the block's triangle centroids into patches of at most PT_MAX triangles, a
-// patch split again while it touches more than PCOLS vertices.  A vertex whose incident triangles
+// coordinate bisection of the block's triangle centroids into patches of at most PT_MAX triangles (fewer in
+// small systems), a patch split again while it touches more than PCOLS vertices.  A vertex whose incident triangles
 // all lie in one patch is a complete column of that patch (the tile writes its G column); any other
 // vertex is partial: each patch touching it writes a halo column, in increasing patch order, and the
 // halo reduction sums them into its G column.  mbase and pbase: the element offsets of each block's G
 // block and row partials (batches: the packed layout; a single system: 0).
 static void build_patches(int64_t N, int64_t M, const double* verts, HostTopo& h, const std::vector<int64_t>& blocks,
-                          const std::vector<long long>& mbase) {
+                          const std::vector<long long>& mbase, bool mirror) {
     std::vector<double> cen((size_t)(3 * M));
     for (int64_t j = 0; j < M; ++j)
         for (int d = 0; d < 3; ++d) {
@@ -141,9 +141,9 @@ static void build_patches(int64_t N, int64_t M, const double* verts, HostTopo& h
             return (int)(std::unique(vs.begin(), vs.end()) - vs.begin());
         }
         static void go(std::vector<int>& idx, int lo, int hi, const std::vector<double>& xyz,
-                       const std::vector<int>& tri, std::vector<std::vector<int>>& out) {
+                       const std::vector<int>& tri, int cap, std::vector<std::vector<int>>& out) {
             const int n = hi - lo;
-            if (n <= PT_MAX && (n == 1 || ncols(tri, idx.data() + lo, idx.data() + hi) <= PCOLS)) {
+            if (n <= cap && (n == 1 || ncols(tri, idx.data() + lo, idx.data() + hi) <= PCOLS)) {
                 out.emplace_back(idx.begin() + lo, idx.begin() + hi);
                 return;
             }
@@ -158,12 +158,12 @@ static void build_patches(int64_t N, int64_t M, const double* verts, HostTopo& h
                 if (mx[d] - mn[d] > mx[ax] - mn[ax]) ax = d;
             std::stable_sort(idx.begin() + lo, idx.begin() + hi,
                              [&](int a, int b) { return xyz[3 * (size_t)a + ax] < xyz[3 * (size_t)b + ax]; });
-            // full patches of PT_MAX on the left where the count allows; halves once a patch of
-            // PT_MAX or fewer triangles is still too wide
-            const int nparts = (n + PT_MAX - 1) / PT_MAX;
-            const int left = nparts > 1 ? (nparts / 2) * PT_MAX : n / 2;
-            go(idx, lo, lo + left, xyz, tri, out);
-            go(idx, lo + left, hi, xyz, tri, out);
+            // full patches of cap triangles on the left where the count allows; halves once a patch of
+            // cap or fewer triangles is still too wide
+            const int nparts = (n + cap - 1) / cap;
+            const int left = nparts > 1 ? (nparts / 2) * cap : n / 2;
+            go(idx, lo, lo + left, xyz, tri, cap, out);
+            go(idx, lo + left, hi, xyz, tri, cap, out);
         }
     };
     const int nb = (int)blocks.size() - 1;
@@ -173,6 +173,16 @@ static void build_patches(int64_t N, int64_t M, const double* verts, HostTopo& h
         for (int64_t v = blocks[(size_t)b]; v < blocks[(size_t)b + 1]; ++v) blk_of_vert[(size_t)v] = b;
     std::vector<std::vector<int>> btri((size_t)nb);
     for (int64_t j = 0; j < M; ++j) btri[(size_t)blk_of_vert[(size_t)h.tri[(size_t)(3 * j)]]].push_back((int)j);
+    long long pairs = 0;  // (row tile, triangle)
+    for (int b = 0; b < nb; ++b)
+        pairs += (long long)btri[(size_t)b].size() * ((blocks[(size_t)b + 1] - blocks[(size_t)b] + PATCH_ROWS - 1) / PATCH_ROWS);
+    // Patches of PT_MAX triangles cost the least per pair, but a small system then leaves SMs without a tile, and a
+    // tile's triangles are a serial chain: about three tiles per SM, four with the wall image (whose pairs take
+    // nearly twice the time).  Assembly in all, us, with 32 triangles and with this rule: N = 162: 27.6, 14.7;
+    // 492: 29.0, 20.6; 1002: 40.7, 38.0; with the image 812: 58.0, 45.6; 1442: 93.9, 90.2.  Below five the columns'
+    // sums over the patches take what the tiles gain (N = 492: 22.4 at four).
+    const int tiles = (mirror ? 4 : 3) * 148;
+    const int cap = (int)std::min<long long>(PT_MAX, std::max<long long>(5, (pairs + tiles - 1) / tiles));
     h.pinfo.clear();
     h.patch_tri.clear();
     h.patch_slot.clear();
@@ -186,7 +196,7 @@ static void build_patches(int64_t N, int64_t M, const double* verts, HostTopo& h
         h.max_block_n = std::max(h.max_block_n, n);
         std::vector<std::vector<int>> leaves;
         auto& idx = btri[(size_t)b];
-        if (!idx.empty()) Rec::go(idx, 0, (int)idx.size(), cen, h.tri, leaves);
+        if (!idx.empty()) Rec::go(idx, 0, (int)idx.size(), cen, h.tri, cap, leaves);
         const int np = (int)leaves.size();
         h.blk_npatch[(size_t)b] = np;
         for (int lp = 0; lp < np; ++lp) {
@@ -856,7 +866,7 @@ int bem_set_mesh(bem_ctx* c, int64_t N, const double* verts, int64_t M, const in
     // a rejected mesh leaves the current one in place
     int rc = build_topology(N, M, trigs, verts, h, c->err);
     if (rc) return rc;
-    build_patches(N, M, verts, h, {0, N}, {0});
+    build_patches(N, M, verts, h, {0, N}, {0}, c->prm.mirror != 0);
     cudaStreamSynchronize(c->stream);
     free_all(*c, true);
     rc = alloc_mesh(*c, N, M, h);
@@ -937,7 +947,7 @@ int bem_set_mesh_blocks(bem_ctx* c, int64_t N, const double* verts, int64_t M, c
     {  // triangle patches of the G-only assembly, block by block
         std::vector<long long> mbases((size_t)nblocks);
         for (int b = 0; b < nblocks; ++b) mbases[(size_t)b] = C.h_blk[(size_t)b].mbase;
-        build_patches(N, M, verts, h, voff, mbases);
+        build_patches(N, M, verts, h, voff, mbases, C.prm.mirror != 0);
         long long ppb = 0;
         for (int b = 0; b < nblocks; ++b) {
             BlockInfo& B = C.h_blk[(size_t)b];
