@@ -821,63 +821,69 @@ static_assert(PR_SING + 9 <= PREC, "the record holds the singular pairs");
 // the 7-point rule's index (c_quv) of the points in this order
 __constant__ int c_porder[7] = {0, 3, 1, 2, 6, 4, 5};
 
-// Threads [0, M): the records; without the wall image threads [M, 4M) also evaluate the singular
-// pairs, one (triangle, corner) each (Integrator.cpp:13-41), into the record's singular slots.
+// A CTA takes PR_TRI triangles: without the wall image one warp their records and three the singular pairs, one
+// (triangle, corner) per thread (Integrator.cpp:13-41); with it each thread a record.  The records are put together
+// in shared memory and written as one run: as 8-byte stores 320 bytes apart they took 186 us for the 618 thousand
+// triangles of a sweep, now 74 (the singular pairs' divisions and roots).
 template <bool MIRROR>
-__global__ void k_patch_records(int M, const double* __restrict__ x, const double* __restrict__ phi,
-                                const int* __restrict__ tri, const int* __restrict__ ptri,
-                                const int* __restrict__ pslot, double* __restrict__ prec) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!MIRROR && q >= M) {
-        if (q >= 4 * M) return;
-        const int p = (q - M) / 3, k = (q - M) - 3 * p;
+constexpr int PR_TRI = MIRROR ? 128 : 32;
+template <bool MIRROR>
+__global__ void __launch_bounds__(128) k_patch_records(int M, const double* __restrict__ x, const double* __restrict__ phi,
+                                                       const int* __restrict__ tri, const int* __restrict__ ptri,
+                                                       const int* __restrict__ pslot, double* __restrict__ prec) {
+    constexpr int TRI = PR_TRI<MIRROR>, LD = PREC + 1;  // odd: no bank conflicts across triangles
+    extern __shared__ double srecs[];                   // [TRI][LD]
+    const int p0 = blockIdx.x * TRI, l = threadIdx.x % TRI, p = p0 + l;
+    double* r = srecs + l * LD;
+    if (p < M) {
         const int t = ptri[p];
-        const int ta = tri[3 * t], tb = tri[3 * t + 1], tc = tri[3 * t + 2];
-        double gg[3], hh[3];
-        singular_sums<false>(x, ta, tb, tc, k, gg, hh);  // gg[m]: the column of vertex (m + k) % 3
-        double* r = prec + (size_t)p * PREC + PR_SING;
+        const int ia = tri[3 * t], ib = tri[3 * t + 1], ic = tri[3 * t + 2];
+        if (!MIRROR && threadIdx.x >= TRI) {
+            const int k = threadIdx.x / TRI - 1;
+            double gg[3], hh[3];
+            singular_sums<false>(x, ia, ib, ic, k, gg, hh);  // gg[m]: the column of vertex (m + k) % 3
 #pragma unroll
-        for (int m = 0; m < 3; ++m) r[3 * k + (m + k) % 3] = gg[m];
-        return;
-    }
-    const int p = q;
-    if (p >= M) return;
-    const int t = ptri[p];
-    const int ia = tri[3 * t], ib = tri[3 * t + 1], ic = tri[3 * t + 2];
-    const double ax = x[3 * ia], ay = x[3 * ia + 1], az = x[3 * ia + 2];
-    const double abx = x[3 * ib] - ax, aby = x[3 * ib + 1] - ay, abz = x[3 * ib + 2] - az;
-    const double acx = x[3 * ic] - ax, acy = x[3 * ic + 1] - ay, acz = x[3 * ic + 2] - az;
-    const double bcx = x[3 * ic] - x[3 * ib], bcy = x[3 * ic + 1] - x[3 * ib + 1], bcz = x[3 * ic + 2] - x[3 * ib + 2];
-    const double nx = aby * bcz - abz * bcy, ny = abz * bcx - abx * bcz, nz = abx * bcy - aby * bcx;
-    const double ab2 = abx * abx + aby * aby + abz * abz, ac2 = acx * acx + acy * acy + acz * acz;
-    const double bc2 = bcx * bcx + bcy * bcy + bcz * bcz;
-    double* r = prec + (size_t)p * PREC;
-    const int sl = pslot[p], col = PATCH_ROWS * (int)sizeof(double);
-    *reinterpret_cast<int4*>(r) = make_int4((sl & 255) * col, (sl >> 8 & 255) * col, (sl >> 16 & 255) * col, 0);
-    r[2] = ax;
-    r[3] = ay;
-    r[4] = az;
-    r[5] = 2.0 * abx;
-    r[6] = 2.0 * aby;
-    r[7] = 2.0 * abz;
-    r[8] = 2.0 * acx;
-    r[9] = 2.0 * acy;
-    r[10] = 2.0 * acz;
-    r[11] = ab2;
-    r[12] = ac2;
-    r[13] = -nx;
-    r[14] = -ny;
-    r[15] = -nz;
-    r[16] = sqrt(nx * nx + ny * ny + nz * nz);
-    const double fa = phi[ia], fb = phi[ib], fc = phi[ic];
+            for (int m = 0; m < 3; ++m) r[PR_SING + 3 * k + (m + k) % 3] = gg[m];
+        } else {
+            const double ax = x[3 * ia], ay = x[3 * ia + 1], az = x[3 * ia + 2];
+            const double abx = x[3 * ib] - ax, aby = x[3 * ib + 1] - ay, abz = x[3 * ib + 2] - az;
+            const double acx = x[3 * ic] - ax, acy = x[3 * ic + 1] - ay, acz = x[3 * ic + 2] - az;
+            const double bcx = x[3 * ic] - x[3 * ib], bcy = x[3 * ic + 1] - x[3 * ib + 1], bcz = x[3 * ic + 2] - x[3 * ib + 2];
+            const double nx = aby * bcz - abz * bcy, ny = abz * bcx - abx * bcz, nz = abx * bcy - aby * bcx;
+            const double ab2 = abx * abx + aby * aby + abz * abz, ac2 = acx * acx + acy * acy + acz * acz;
+            const double bc2 = bcx * bcx + bcy * bcy + bcz * bcz;
+            const int sl = pslot[p], col = PATCH_ROWS * (int)sizeof(double);
+            r[0] = __hiloint2double((sl >> 8 & 255) * col, (sl & 255) * col);
+            r[1] = __hiloint2double(0, (sl >> 16 & 255) * col);
+            r[2] = ax;
+            r[3] = ay;
+            r[4] = az;
+            r[5] = 2.0 * abx;
+            r[6] = 2.0 * aby;
+            r[7] = 2.0 * abz;
+            r[8] = 2.0 * acx;
+            r[9] = 2.0 * acy;
+            r[10] = 2.0 * acz;
+            r[11] = ab2;
+            r[12] = ac2;
+            r[13] = -nx;
+            r[14] = -ny;
+            r[15] = -nz;
+            r[16] = sqrt(nx * nx + ny * ny + nz * nz);
+            const double fa = phi[ia], fb = phi[ib], fc = phi[ic];
 #pragma unroll
-    for (int e = 0; e < 7; ++e) {
-        const int k = c_porder[e];
-        const double u = c_quv[k][0], v = c_quv[k][1], l0 = 1.0 - u, l1 = u - v;
-        r[PR_W + e] = -(l0 * l1 * ab2 + l0 * v * ac2 + l1 * v * bc2);
-        r[PR_PHI + e] = c_qc[k][0] * fa + c_qc[k][1] * fb + c_qc[k][2] * fc;
-        if (MIRROR) r[PR_YX + e] = ax + u * abx + v * bcx;
+            for (int e = 0; e < 7; ++e) {
+                const int k = c_porder[e];
+                const double u = c_quv[k][0], v = c_quv[k][1], l0 = 1.0 - u, l1 = u - v;
+                r[PR_W + e] = -(l0 * l1 * ab2 + l0 * v * ac2 + l1 * v * bc2);
+                r[PR_PHI + e] = c_qc[k][0] * fa + c_qc[k][1] * fb + c_qc[k][2] * fc;
+                if (MIRROR) r[PR_YX + e] = ax + u * abx + v * bcx;
+            }
+        }
     }
+    __syncthreads();
+    const int words = min(TRI, M - p0) * PREC;
+    for (int e = threadIdx.x; e < words; e += 128) prec[(size_t)p0 * PREC + e] = srecs[e / PREC * LD + e % PREC];
 }
 
 // One regular (row, triangle) pair: g_k (to be scaled by the area), and hb takes the row's share of b,
@@ -1207,11 +1213,13 @@ void launch_assemble_g(Ctx& c, const double* x, const double* phi, double* b, cu
     }
     // records (and, without the wall image, the singular pairs)
     if (c.prm.mirror)
-        KLAUNCH(), k_patch_records<true><<<(M + 127) / 128, 128, 0, s>>>(M, x, phi, T.tri, T.patch_tri,
-                                                                          T.patch_slot, c.prec);
+        KLAUNCH(), k_patch_records<true><<<(M + PR_TRI<true> - 1) / PR_TRI<true>, 128,
+                                           sizeof(double) * PR_TRI<true> * (PREC + 1), s>>>(M, x, phi, T.tri, T.patch_tri,
+                                                                                          T.patch_slot, c.prec);
     else
-        KLAUNCH(), k_patch_records<false><<<(4 * M + 127) / 128, 128, 0, s>>>(M, x, phi, T.tri, T.patch_tri,
-                                                                               T.patch_slot, c.prec);
+        KLAUNCH(), k_patch_records<false><<<(M + PR_TRI<false> - 1) / PR_TRI<false>, 128,
+                                            sizeof(double) * PR_TRI<false> * (PREC + 1), s>>>(
+                       M, x, phi, T.tri, T.patch_tri, T.patch_slot, c.prec);
     constexpr size_t sm = patch_smem<PATCH_ROWS>();
     if (c.prm.mirror)
         KLAUNCH(), k_assemble_patch<true, PATCH_ROWS, 3><<<T.nwork, PATCH_ROWS, sm, s>>>(
