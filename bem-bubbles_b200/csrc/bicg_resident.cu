@@ -26,8 +26,9 @@
 // N = 812 with the wall image: 0.23 ms (1.13), N = 1442: 0.35 ms (1.66), N = 1962: 0.54 ms.
 //
 // Matrix streamed: bound by the two reads of the matrix per iteration.  Each thread copies two rows of its
-// columns (16 bytes) into a ring of its own in shared memory, 12 copies ahead (98 KB in flight per SM, no
-// registers held, no barrier: a thread reads only what it copied), and the copies run on through the exchanges.
+// columns (16 bytes) into a ring of its own in shared memory, 12 copies ahead in groups of four (98 KB in flight
+// per SM, no registers held, no barrier: a thread reads only what it copied), and the copies run on through the
+// exchanges.  One copy per group took 1 to 3 % longer up to N = 4096.
 // 64 MB of the matrix are marked to stay in L2 (evict_last, the rest evict_first).  Per iteration: N = 4002:
 // 38 us (6.7 TB/s of matrix reads) against 91 us for k_pbicg; 42 us without the marks, 47 us with 100 MB marked.
 // With loads into registers instead of the ring 48 us; with a TMA ring of row slabs 71 us (a slab's rows are
@@ -46,12 +47,13 @@ namespace bemb {
 
 namespace {
 
+constexpr int RB_U = 4;                // streamed: columns per group of copies
 constexpr int RB_D8 = 12, RB_D12 = 8;  // streamed: copies in flight per thread, up to 4096 and 6144 unknowns
 constexpr double RB_EPS = 2.220446049250313080847e-16;
 
 struct RBArgs {
     int n, ld, rows, nv, npart, maxit;  // rows per CTA; doubles of the input vector and of the row partials
-    int nk;                            // streamed: columns per thread
+    int nk;                            // streamed: groups of RB_U columns per thread
     float keep;                        // streamed: share of the matrix to keep in L2
     const double* A;
     const double* b;
@@ -85,21 +87,21 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
     const double* next = a.A + (size_t)min(c, n - 1) * a.ld + row0 + min(i, nr - 1);
     int nextj = c, slot = 0;
     auto advance = [&](int d) {
-        if (active) {
-            ring_copy(ring + d * RB_T, next, nextj < n, pol);
-            nextj += cstep;
-            next += (size_t)cstep * a.ld;
-            if (nextj >= a.nk * cstep) {  // the next product
-                nextj -= a.nk * cstep;
-                next -= (size_t)a.nk * cstep * a.ld;
-            }
-        }
+#pragma unroll
+        for (int u = 0; u < RB_U; ++u)
+            if (active) ring_copy(ring + (d + u) * RB_T, next + (size_t)u * cstep * a.ld, nextj + u * cstep < n, pol);
         asm volatile("cp.async.commit_group;" ::: "memory");
+        nextj += RB_U * cstep;
+        next += (size_t)RB_U * cstep * a.ld;
+        if (nextj >= a.nk * RB_U * cstep) {  // the next product
+            nextj -= a.nk * RB_U * cstep;
+            next -= (size_t)a.nk * RB_U * cstep * a.ld;
+        }
     };
     if (ST) {
         asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(pol) : "f"(a.keep));
 #pragma unroll
-        for (int d = 0; d < D; ++d) advance(d);
+        for (int d = 0; d < D; d += RB_U) advance(d);
     }
     // the thread's entries of the own rows (not ST): columns c + q cstep, the first M in registers, the others
     // (columns from M cstep on) in shared memory
@@ -164,15 +166,23 @@ __global__ void __launch_bounds__(RB_T, 1) k_bicg_resident(const RBArgs a) {
             // the own rows of A vec
             double acc[4] = {0.0, 0.0, 0.0, 0.0};
             if (ST) {
-                const double* vc = vec + c;
                 for (int k = 0; k < a.nk; ++k) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(ST ? D - 1 : 0) : "memory");
-                    const double2 v = ring[slot * RB_T];
-                    const double xv = vc[k * cstep];
-                    acc[0] = fma(v.x, xv, acc[0]);
-                    acc[1] = fma(v.y, xv, acc[1]);
+                    asm volatile("cp.async.wait_group %0;" ::"n"(ST ? D / RB_U - 1 : 0) : "memory");
+                    const double* vc = vec + c + k * RB_U * cstep;
+                    double2 v[RB_U];
+                    double xv[RB_U];
+#pragma unroll
+                    for (int u = 0; u < RB_U; ++u) {
+                        v[u] = ring[(slot + u) * RB_T];
+                        xv[u] = vc[u * cstep];
+                    }
+#pragma unroll
+                    for (int u = 0; u < RB_U; ++u) {
+                        acc[0] = fma(v[u].x, xv[u], acc[0]);
+                        acc[1] = fma(v[u].y, xv[u], acc[1]);
+                    }
                     advance(slot);
-                    slot = slot + 1 == D ? 0 : slot + 1;
+                    slot = slot + RB_U == D ? 0 : slot + RB_U;
                 }
                 if (active) {
                     part[i * (cstep + 1) + c] = acc[0];
@@ -320,11 +330,11 @@ int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaS
         a.rows = ((n + sms - 1) / sms + 1) & ~1;  // even: a copy takes two rows
         grid = (n + a.rows - 1) / a.rows;
         const int cstep = RB_T / (a.rows / 2), D = K <= 8 ? RB_D8 : RB_D12;
-        a.nk = (n + cstep - 1) / cstep;
-        a.nv = (a.nk * cstep + 1) & ~1;
+        a.nk = (n + RB_U * cstep - 1) / (RB_U * cstep);
+        a.nv = (a.nk * RB_U * cstep + cstep + 1) & ~1;  // idle threads read a little past their columns
         a.npart = a.rows * (cstep + 1);
         smem = sizeof(double) * ((size_t)2 * D * RB_T + a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS);
-        if (smem > RB_SMEM || a.rows > 2 * RB_T || a.nk < D || !c.LU) return BEM_ERR_STATE;
+        if (smem > RB_SMEM || a.rows > 2 * RB_T || !c.LU) return BEM_ERR_STATE;
         // the part of the matrix that the L2 can hold beside the stream
         a.keep = (float)std::min(1.0, RB_KEEP / (8.0 * n * n));
         if (n % 2 || reinterpret_cast<uintptr_t>(A) % 16) {  // copies of 16 bytes: a matrix with an even stride
