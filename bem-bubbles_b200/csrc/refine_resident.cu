@@ -5,10 +5,10 @@
 // What bounds it: the reads of G and X, 12 N^2 bytes per step.  As separate launches a step's two GEMVs each
 // pay their ramp, the tail of the column splits and, at small sizes, mostly the launch; the number of steps had
 // to be guessed, with gated extra steps behind it.  Here a thread copies 16 bytes (two rows of G or four of X)
-// per column into a ring of its own, RF_D copies ahead across the products and exchanges, X marked to stay in L2
-// (64 MB at N = 4002) and G to pass through.  Two exchanges per step (bicg_resident.cu describes them).
-// Measured (B200) per solve of two or three steps, against the separate launches: N = 4002: 207 us (409),
-// N = 1002: 37 us (about 105, with the gaps).
+// per column into a ring of its own, RF_D copies ahead across the products and exchanges, RB_KEEP bytes marked to
+// stay in L2.  Two exchanges per step (bicg_resident.cu describes them).
+// Measured (B200) per solve, against the separate launches: N = 4002, five steps: 182 us (409); N = 1002, three to
+// four steps: 38 us (about 105, with the gaps).
 // In a batch a team of CTAs takes one block after another, so that no stage waits for the slowest block between
 // its products: four stages of 24 blocks of 362 to 1442 unknowns 5.16 -> 4.16 ms, of 256 of them 53.1 -> 51.0 ms
 // (the matrices then come from HBM either way: 31 B per clock and SM).
@@ -44,7 +44,7 @@ struct RRule {
     int kmax;
     double tol, strict, slow;  // stop at strict tol, or one step past tol; or when a step above 1000 tol
     long long wait_limit;      // contracts by no more than slow
-    float keep;                // share of G to keep in L2 beside X
+    float keep_g, keep_x;      // shares of G and X to keep in L2
 };
 
 // The refinement of one system by the CTAs that share it.  record(step, rel, last) is called by every thread
@@ -62,8 +62,8 @@ __device__ bool refine_system(const RSys& a, const RRule& q, double* smem, int n
     const int px = rows / 4, cx = RB_T / px, ix = tid % px * 4, jx = tid / px, nkx = (n + RF_U * cx - 1) / (RF_U * cx);
     const bool ong = jg < cg && ig < nr, onx = jx < cx && ix < nr;
     uint64_t polg, polx;
-    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(polg) : "f"(q.keep));
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(polx));
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(polg) : "f"(q.keep_g));
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(polx) : "f"(q.keep_x));
     // the stream: products with G and X in turn, columns jg + k cg and jx + k cx, RF_U at a time
     const double* gsrc = a.A + (size_t)min(jg, n - 1) * a.ldg + (ong ? row0 + ig : 0);
     const float* xsrc = a.X + (size_t)min(jx, n - 1) * a.ldx + (onx ? row0 + ix : 0);
@@ -366,8 +366,10 @@ static int rr_round(Ctx& c, RSys& a, const RRule& q, double* out, unsigned long 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.device);
     if (!coop) return BEM_ERR_CUDA;
-    // 16 rows as in bicg_resident.cu, more where the SMs run out; a multiple of four (X's copies)
-    a.rows = std::max(16, ((a.n + sms - 1) / sms + 3) & ~3);
+    // 16 rows as in bicg_resident.cu, more where the SMs run out; a multiple of eight, so that a CTA's part of a
+    // column of X is whole sectors: 32 rows on 126 SMs at N = 4002 39.4 us per step with the first residual's
+    // share, 28 rows on 143 SMs 41.0; N = 5292: 69.1 and 71.9; N = 4842: 63.9 and 63.0
+    a.rows = std::max(16, ((a.n + sms - 1) / sms + 7) & ~7);
     const int grid = (a.n + a.rows - 1) / a.rows;
     int nv = 0, npart = 0;
     rr_sizes(a.n, a.rows, &nv, &npart);
@@ -387,10 +389,12 @@ static int rr_round(Ctx& c, RSys& a, const RRule& q, double* out, unsigned long 
     return BEM_OK;
 }
 
-// The share of G that the L2 holds beside X.
-static float rr_keep(int n) {
-    const double nn = (double)n * n;
-    return (float)std::max(0.0, std::min(1.0, (RB_KEEP - 4.0 * nn) / (8.0 * nn)));
+// A rule with the shares of G and X to keep in L2: RB_KEEP bytes, G first.  At N = 4002 with rows of 32, per step:
+// 64 MB of G 33.7 us, 32 MB of G and of X 34.6, X alone 36.6, all of X and 32 MB of G 37.8.
+static RRule rr_rule(const Ctx& c, int n, int kmax, double tol, double strict, double slow) {
+    const double g = 8.0 * n * n, x = 4.0 * n * n;
+    return {kmax, tol, strict, slow, c.wait_limit, (float)std::min(1.0, RB_KEEP / g),
+            (float)std::max(0.0, std::min(1.0, (RB_KEEP - g) / x))};
 }
 
 // One round of at most kmax steps from x; out (3 + kmax + 1 doubles on the device, as k_refine_resident leaves
@@ -415,7 +419,7 @@ int refine_resident(Ctx& c, const double* A, const double* b, double* x, const d
     a.x = x;
     // a tenth of the tolerance, or one step past it: the last step is cheap, and a solve that only just meets
     // the tolerance would leave the solution less exact than the rounds of separate launches do
-    const RRule q{kmax, tol, tol >= 1e-13 ? 0.1 : 1.0, slow, c.wait_limit, rr_keep(n)};
+    const RRule q = rr_rule(c, n, kmax, tol, tol >= 1e-13 ? 0.1 : 1.0, slow);
     return rr_round(c, a, q, out, number, s);
 }
 
@@ -460,7 +464,7 @@ int refine_resident_transposed(Ctx& c, const double* G, const double* b, double*
         BEM_CUDA(c, cudaMemsetAsync(y, 0, sizeof(double) * n, s));
     }
     // the separate launches always run six steps: two orders below the tolerance, or one step past it
-    const RRule q{kmax, tol, tol >= 1e-13 ? 0.01 : 1.0, INFINITY, c.wait_limit, rr_keep(n)};
+    const RRule q = rr_rule(c, n, kmax, tol, tol >= 1e-13 ? 0.01 : 1.0, INFINITY);
     return rr_round(c, a, q, out, number, s);
 }
 
@@ -554,7 +558,8 @@ int refine_batch_inverse(Ctx& c, int b, cudaStream_t s) {
 int refine_batch(Ctx& c, const double* A, const double* b, double* x, int kmax, double tol, double* err, cudaStream_t s) {
     BRArgs a{c.blk, c.blist, c.boff, c.bxoff, A, c.Xb, c.Xbpad, b, x, reinterpret_cast<ulonglong2*>(c.bslots),
              (long long)c.topo.N, c.bnumber, c.bstat, err, c.bconv, c.bteam, c.bnv, c.bnpart};
-    RRule q{kmax, tol, 1.0, INFINITY, c.wait_limit, 1.0f};
+    RRule q{kmax, tol, 1.0, INFINITY, c.wait_limit, 1.0f, 1.0f};
+
     KLAUNCH(), k_next_number<<<1, 1, 0, s>>>(c.bnumber);
     void* args[] = {&a, &q};
     KLAUNCH();
