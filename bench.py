@@ -664,7 +664,7 @@ def run_lu(args):
                                "factorisation and triangular solves, device-resident G (the copy-in excluded)",
                    "solver": "lu"},
         "scaled_residual": res,
-        "roofline": {"bound": "fp64-fma", "kernel": "k_lu_panel_cluster + k_lu_update + k_lu_trsm + k_trsv_*",
+        "roofline": {"bound": "fp64-fma", "kernel": "k_lu_panel_cluster + k_lu_update + k_lu_swap_trsm + k_lu_back",
                      "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
                      "flops_per_solve": flops},
         "gpu_launches": int(prof.kernel_launches / max(1, prof.solve_calls)),

@@ -76,9 +76,11 @@ typedef struct {
  * H.  Both give the same G and b to rounding; for comparison. */
 #define BEM_FLAG_STEP_ASSEMBLE_H 4
 /* bem_params.flags: run each round of BEM_SOLVER_MIXED's refinement steps as one cooperative kernel
- * with grid barriers instead of separate GEMV launches (the same tiles and summation order:
+ * with grid barriers over the tiles of the separate GEMV launches (the same summation order:
  * bit-identical results, with BEM_FLAG_NO_IR_GATE).  Measured slower than the separate launches on
- * B200 (0.36 against 0.27 ms per solve at N = 4002), so it is not the default. */
+ * B200 (0.36 against 0.27 ms per solve at N = 4002), and those slower than the default for N <= 6144,
+ * a cooperative launch whose vectors stay on the SMs and whose convergence test is on the device
+ * (0.21 ms).  For comparison. */
 #define BEM_FLAG_REFINE_PERSISTENT 8
 /* bem_params.flags: how BEM_SOLVER_MIXED builds its approximate inverse from scratch.  By default
  * (neither flag) large systems (N >= BEM_GJ_MIN_N) use blocked Gauss-Jordan elimination with row
@@ -87,8 +89,9 @@ typedef struct {
 #define BEM_FLAG_INVERSE_GJ 16
 #define BEM_FLAG_INVERSE_NS 32
 #define BEM_GJ_MIN_N 8192
-/* bem_params.flags: no gated extra steps in the first round of BEM_SOLVER_MIXED's refinement.  By
- * default that round issues one or two steps beyond its estimate whose GEMVs a device-side check of
+/* bem_params.flags: separate GEMV launches in BEM_SOLVER_MIXED's refinement at every N, and no gated
+ * extra steps in the first round.  By default, where the rounds are separate launches (N > 6144, or no
+ * cooperative launch), that round issues one or two steps beyond its estimate whose GEMVs a device-side check of
  * the convergence rule skips once it holds, so a short estimate does not cost a second round (a
  * read-back of the residual norms by the host and a new enqueue).  With the flag a round issues its
  * estimate only, as the cooperative round kernel of BEM_FLAG_REFINE_PERSISTENT does. */
@@ -277,8 +280,8 @@ typedef struct {
                                  singular G, e.g. a bubble cut by its own wall image) */
     int64_t total_iters;      /* iterations of every iterative solve since creation (refinement steps of
                                  the mixed path, including its GMRES hand-overs; BiCGSTAB iterations) */
-    int64_t wait_expired;     /* bounded grid-barrier waits of the persistent kernels (BiCGSTAB, LU
-                                 panel) that gave up; each sent the context to the multi-kernel form */
+    int64_t wait_expired;     /* bounded waits of the persistent kernels (BiCGSTAB, refinement, LU) that
+                                 gave up; each sent the context to the multi-kernel form */
     int64_t gj_inverses;      /* approximate inverses of the mixed path built by the tensor-core
                                  Gauss-Jordan elimination (the rest by Newton-Schulz from scratch) */
     int64_t ir_rounds;        /* rounds of refinement steps of the mixed path since creation (each ends
@@ -287,8 +290,8 @@ typedef struct {
 int bem_get_stats(bem_ctx* ctx, bem_stats* s);
 
 /* Bound, in SM clock cycles, of every grid-wide barrier or exchange wait of the persistent kernels (the
- * cooperative BiCGSTAB forms, the cooperative refinement round, the row-distributed LU panel) and of the
- * LU cluster panel's exchange waits.  Default 2e9 (about a second at the B200's clock).  A wait that
+ * cooperative BiCGSTAB forms, the cooperative refinement rounds of a system and of a batch, the
+ * row-distributed LU panel) and of the LU cluster panel's and back substitution's waits.  Default 2e9 (about a second at the B200's clock).  A wait that
  * runs out makes the kernel set its error word and return; the host reads it, counts it in
  * bem_stats.wait_expired and finishes the solve with the multi-kernel form (for the LU: the
  * single-CTA panel), which the context keeps for the rest of its life.  No counterpart in the reference (its solves
