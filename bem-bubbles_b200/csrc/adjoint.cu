@@ -552,8 +552,6 @@ static int adj_alloc(Ctx& c, int steps) {
             (rc = dalloc(c, &w.S, (size_t)c.topo.nparts + 1)) || (rc = dalloc(c, &w.red, (size_t)nbk(N, 8) * 16 + 64)) ||
             (rc = dalloc(c, &w.tsave, 2)) || (rc = dalloc(c, &w.iox, 3 * N)) || (rc = dalloc(c, &w.iop, N)))
             return rc;
-        if (refine_resident_fits(c) && dalloc(c, &w.xt, N * ((N + 3) & ~(size_t)3)))
-            cudaGetLastError();  // no memory for it: the separate launches
     }
     w.N = (int64_t)N;
     w.cap = cap;
@@ -713,6 +711,8 @@ int adjoint_record(Ctx& c, double dt, int steps) {
     AdjWork& w = c.adj;
     cudaStream_t s = c.stream;
     const int64_t N = c.topo.N;
+    if (!w.xt && refine_resident_fits(c) && dalloc(c, &w.xt, (size_t)N * ((N + 3) & ~(int64_t)3)))
+        cudaGetLastError();  // no memory for it: the separate launches
     int flag = 0;
     BEM_CUDA(c, cudaMemsetAsync(c.flag + 2, 0, sizeof(int), s));
     KLAUNCH(), k_any_below<<<nbk(N, 256), 256, 0, s>>>((int)N, c.x, c.prm.nopen_eps, c.flag + 2);
