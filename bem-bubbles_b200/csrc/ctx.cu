@@ -715,9 +715,8 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         (rc = dalloc(c, &c.bp, nrow_part)) || (!c.batch && (rc = dalloc(c, &c.gp, nrow_part))) || (rc = dalloc(c, &c.vol, (size_t)h.nparts + 1)) ||
         (rc = dalloc(c, &c.vol_part, (size_t)h.nparts * 64)) || (rc = dalloc(c, &c.vol_cnt, (size_t)h.nparts)) ||
         (rc = dalloc(c, &c.part, (size_t)ncs * n)) || (rc = dalloc(c, &c.cnt, (n + 255) / 256 + 1)) ||
-        (rc = dalloc(c, &c.red, (size_t)(c.gmres_m + 8) * VBLK + 4096)) || (rc = dalloc(c, &c.piv, n)) || (!c.batch && (rc = dalloc(c, &c.lu_x, 2 * n))) ||
+        (rc = dalloc(c, &c.red, (size_t)(c.gmres_m + 8) * VBLK + 4096)) || (rc = dalloc(c, &c.piv, n)) || (!c.batch && (rc = dalloc(c, &c.lu_x, 2 * n + rbicg_words(N)))) ||
         (rc = dalloc(c, &c.hcol, (size_t)2 * (c.gmres_m + 2) + 8)) || (rc = dalloc(c, &c.pbicg, pbicg_words(N))) ||
-        (!c.batch && (rc = dalloc(c, &c.rbicg, rbicg_words(N)))) ||
         (!c.batch && (rc = dalloc(c, &c.lu_aux, lu_panel_words()))) ||
         (!c.batch && (rc = dalloc(c, &c.psih, (size_t)PRED_DEPTH * 4 * n))) ||
         (!c.batch && (rc = dalloc(c, &c.psih_t, (size_t)PRED_CNT + 1))))
@@ -738,8 +737,8 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         if ((rc = alloc_mixed(c))) return rc;
     }
     BEM_CUDA(c, cudaMemset(c.cnt, 0, sizeof(unsigned) * ((n + 255) / 256 + 1)));
-    if (c.lu_x) BEM_CUDA(c, cudaMemset(c.lu_x, 0, sizeof(double) * 2 * n));
-    if (c.rbicg) BEM_CUDA(c, cudaMemset(c.rbicg, 0, sizeof(double) * rbicg_words(N)));
+    if (c.lu_x) BEM_CUDA(c, cudaMemset(c.lu_x, 0, sizeof(double) * (2 * n + rbicg_words(N))));
+    c.rbicg = c.lu_x ? c.lu_x + 2 * n : nullptr;  // slots of 16 bytes
     BEM_CUDA(c, cudaMemset(c.vol_cnt, 0, sizeof(unsigned) * (size_t)h.nparts));
     BEM_CUDA(c, cudaMemset(c.phi, 0, sizeof(double) * n));
     BEM_CUDA(c, cudaMemset(c.psi, 0, sizeof(double) * n));
@@ -800,12 +799,12 @@ int bem_create(bem_ctx** out, int device, const bem_params* p) {
         bem_default_params(&c->prm);
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void**)&c->sc, sizeof(DevScalars)) != cudaSuccess ||
-        cudaMallocHost((void**)&c->h_sc, sizeof(DevScalars)) != cudaSuccess ||
-        cudaMallocHost((void**)&c->h_flag, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMallocHost((void**)&c->h_sc, sizeof(DevScalars) + 2 * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void**)&c->flag, 4 * sizeof(int)) != cudaSuccess) {
         delete c;
         return BEM_ERR_CUDA;
     }
+    c->h_flag = reinterpret_cast<int*>(c->h_sc + 1);
     cudaMemset(c->sc, 0, sizeof(DevScalars));
     cudaMemset(c->flag, 0, 4 * sizeof(int));
     *out = c;
@@ -827,7 +826,6 @@ int bem_destroy(bem_ctx* c) {
     cudaFree(c->sc);
     cudaFree(c->flag);
     cudaFreeHost(c->h_sc);
-    cudaFreeHost(c->h_flag);
     cudaFreeHost(c->h_red);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;

@@ -46,7 +46,7 @@ struct Ctx {
     double* psi = nullptr;  // N
     DevScalars* sc = nullptr;
     DevScalars* h_sc = nullptr;  // pinned mirror
-    int* h_flag = nullptr;       // pinned: the LU's error words
+    int* h_flag = nullptr;       // pinned, behind h_sc: the LU's error words
     double* h_red = nullptr;     // pinned host copy of the mixed solve's residual-norm partials
     size_t h_red_cap = 0;        // its capacity in doubles
 
