@@ -51,7 +51,8 @@ static void free_all(Ctx& c, bool keep_blocks = false) {
     c.asm_err = nullptr;
     c.pbicg = nullptr;
     c.rbicg = nullptr;
-    c.lu_aux = nullptr;
+    c.lu_aux = c.lu_x = nullptr;
+    c.gp = nullptr;
     c.Xinv = c.Xpad = c.Tw = c.G32 = nullptr;
     c.tcp = nullptr;
     c.tc_err = nullptr;
@@ -737,8 +738,10 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         if ((rc = alloc_mixed(c))) return rc;
     }
     BEM_CUDA(c, cudaMemset(c.cnt, 0, sizeof(unsigned) * ((n + 255) / 256 + 1)));
-    if (c.lu_x) BEM_CUDA(c, cudaMemset(c.lu_x, 0, sizeof(double) * (2 * n + rbicg_words(N))));
-    c.rbicg = c.lu_x ? c.lu_x + 2 * n : nullptr;  // slots of 16 bytes
+    if (!c.batch) {
+        BEM_CUDA(c, cudaMemset(c.lu_x, 0, sizeof(double) * (2 * n + rbicg_words(N))));
+        c.rbicg = c.lu_x + 2 * n;  // slots of 16 bytes
+    }
     BEM_CUDA(c, cudaMemset(c.vol_cnt, 0, sizeof(unsigned) * (size_t)h.nparts));
     BEM_CUDA(c, cudaMemset(c.phi, 0, sizeof(double) * n));
     BEM_CUDA(c, cudaMemset(c.psi, 0, sizeof(double) * n));
