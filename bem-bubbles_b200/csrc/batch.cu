@@ -263,17 +263,19 @@ int batch_build_inverses(Ctx& c, cudaStream_t s) {
     return BEM_OK;
 }
 
-// After a batched step: per-block statistics of the last solve to the host.  Blocks whose
-// contraction exceeded 0.02 get a refresh against the G blocks of that last solve; *redo is set when
-// a block missed the tolerance within the refinement steps (the caller re-runs the step).
-int batch_after_step(Ctx& c, cudaStream_t s, bool* redo) {
+// After a batched step, or a velocity evaluation outside one (step false): per-block statistics of the last
+// solve to the host; *redo is set when the caller has to run it again: an exchange wait ran out, or a block
+// missed the tolerance within the refinement steps.  Such a block gets a refresh against the G blocks of that
+// solve, and after a step one whose contraction exceeded 0.02 too.  An evaluation lets a residual that is not
+// finite be: its input was not.
+int batch_check(Ctx& c, cudaStream_t s, bool step, bool* redo) {
     *redo = false;
     double* expired = c.bstat + (size_t)BSTAT_W * c.nblk;
     BEM_CUDA(c, cudaMemcpyAsync(c.bstat_h, c.bstat, sizeof(double) * (BSTAT_W * (size_t)c.nblk + 1), cudaMemcpyDeviceToHost,
                                 s));
     BEM_CUDA(c, cudaStreamSynchronize(s));
     if (c.bstat_h[(size_t)BSTAT_W * c.nblk] != 0.0) {
-        // an exchange wait of the resident refinement ran out: the step starts over with the separate launches,
+        // an exchange wait of the resident refinement ran out: all starts over with the separate launches,
         // which the context keeps (and the graph, captured with the other, goes)
         c.stats.wait_expired++;
         c.bteam = 0;
@@ -287,9 +289,9 @@ int batch_after_step(Ctx& c, cudaStream_t s, bool* redo) {
     for (int b = 0; b < c.nblk; ++b) {
         const double* q = c.bstat_h + (size_t)BSTAT_W * b;
         worst = std::max(worst, q[BS_LAST]);
-        const bool ok = q[BS_CONV] != 0.0;
+        const bool ok = q[BS_CONV] != 0.0 || (!step && !std::isfinite(q[BS_LAST]));
         if (!ok) *redo = true;
-        if (!ok || q[BS_RHO] > 0.02) {
+        if (!ok || (step && q[BS_RHO] > 0.02)) {
             int rc = refresh_block(c, c.G, b, s);
             if (rc) return rc;
         }

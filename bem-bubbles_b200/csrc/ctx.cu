@@ -1041,18 +1041,39 @@ int bem_get_block_stats(bem_ctx* c, double* rho, double* rel_residual, int32_t* 
     return batch_block_stats(*c, rho, rel_residual, steps);
 }
 
+// Approximate inverses of the blocks that have none, for positions x.
+static int batch_need_inverses(Ctx& c, const double* x, const double* pot, cudaStream_t s) {
+    bool need = false;
+    for (char v : c.bvalid) need |= !v;
+    if (!need) return BEM_OK;
+    launch_assemble(c, x, pot, c.G, c.H, c.b, s);
+    return batch_build_inverses(c, s);
+}
+
+// Repetitions of a batched solve at most: two with renewed inverses, one after an expired wait (the only one of
+// a context).
+constexpr int BATCH_REDO = 3;
+
+// position_t of a batch outside a step: nothing leaves before the solve's status has been seen.
+static int batch_position_t(Ctx& c, const double* x, double* pot, double* vel, cudaStream_t s) {
+    int rc = batch_need_inverses(c, x, pot, s);
+    if (rc) return rc;
+    for (int attempt = 0;; ++attempt) {
+        bool redo = false;
+        if ((rc = position_t(c, x, pot, vel, s)) || (rc = batch_check(c, s, false, &redo))) return rc;
+        if (!redo) return BEM_OK;
+        if (attempt >= BATCH_REDO)
+            return c.fail(BEM_ERR_NOT_CONVERGED, "batched solve: a block missed the tolerance after refreshing its inverse");
+    }
+}
+
 // Fixed-dt RK4 steps of a batch; with graph != 0 each step is one replay of a captured CUDA graph.
 static int batch_steps(Ctx& c, double dt, int steps, bool graph) {
     cudaStream_t s = c.stream;
     if (c.field_cb) return c.fail(BEM_ERR_STATE, "batches evaluate the pressure field on the device (no callback)");
     int rc = check_negative(c, s);
     if (rc) return rc;
-    bool need = false;
-    for (char v : c.bvalid) need |= !v;
-    if (need) {  // approximate inverses of the blocks that have none, at the current state
-        launch_assemble(c, c.x, c.phi, c.G, c.H, c.b, s);
-        if ((rc = batch_build_inverses(c, s))) return rc;
-    }
+    if ((rc = batch_need_inverses(c, c.x, c.phi, s))) return rc;
     if (graph && (!c.graph_exec || c.graph_dt != dt)) {
         if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
         c.graph_exec = nullptr;
@@ -1090,9 +1111,9 @@ static int batch_steps(Ctx& c, double dt, int steps, bool graph) {
                 return rc;
             }
             bool redo = false;
-            if ((rc = batch_after_step(c, s, &redo))) return rc;
+            if ((rc = batch_check(c, s, true, &redo))) return rc;
             if (!redo) break;
-            if (attempt >= 2)
+            if (attempt >= BATCH_REDO)
                 return c.fail(BEM_ERR_NOT_CONVERGED, "batched solve: a block missed the tolerance after refreshing its inverse");
             // the step starts over from its saved start state (rk4_step copies x, phi to x1, p1 first)
             BEM_CUDA(c, cudaMemcpyAsync(c.x, c.x1, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, s));
@@ -1549,7 +1570,7 @@ static int position_t_host(bem_ctx* c, const double* verts, const double* pot, d
         x = c->xs;
     }
     COPY_IN(c->ps, pot, N);
-    int rc = position_t(*c, x, c->ps, c->k1, c->stream);
+    int rc = c->batch ? batch_position_t(*c, x, c->ps, c->k1, c->stream) : position_t(*c, x, c->ps, c->k1, c->stream);
     if (rc) return rc;
     BEM_CUDA(*c, cudaGetLastError());
     COPY_OUT(vel, c->k1, 3 * N);

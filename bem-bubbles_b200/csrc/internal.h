@@ -315,7 +315,7 @@ int volume_gradient(Ctx& c, double* xbar);
 int batch_mixed_solve(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s);
 int batch_setup_solver(Ctx& c);
 int batch_build_inverses(Ctx& c, cudaStream_t s);
-int batch_after_step(Ctx& c, cudaStream_t s, bool* redo);
+int batch_check(Ctx& c, cudaStream_t s, bool step, bool* redo);
 int batch_block_stats(Ctx& c, double* rho, double* rel, int32_t* steps);
 
 }  // namespace bemb
