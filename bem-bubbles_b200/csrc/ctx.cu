@@ -29,11 +29,16 @@ static void release_reuse(Ctx& c) {
     c.reuse_pos = 0;
 }
 
+// The captured batch step, which holds its launch arguments, goes; the next graph step captures another.
+static void drop_graph(Ctx& c) {
+    if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
+    c.graph_exec = nullptr;
+}
+
 // keep_blocks: the device allocations stay for the next mesh's buffers (see dalloc)
 static void free_all(Ctx& c, bool keep_blocks = false) {
     exporter_release(c);  // writes every queued file first
-    if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
-    c.graph_exec = nullptr;
+    drop_graph(c);
     release_reuse(c);
     if (keep_blocks)
         c.reuse = c.allocs;
@@ -1051,7 +1056,7 @@ static int batch_need_inverses(Ctx& c, const double* x, const double* pot, cudaS
 }
 
 // Repetitions of a batched solve at most: two with renewed inverses, one after an expired wait (the only one of
-// a context).
+// a mesh).
 constexpr int BATCH_REDO = 3;
 
 // position_t of a batch outside a step: nothing leaves before the solve's status has been seen.
@@ -1075,8 +1080,7 @@ static int batch_steps(Ctx& c, double dt, int steps, bool graph) {
     if (rc) return rc;
     if ((rc = batch_need_inverses(c, c.x, c.phi, s))) return rc;
     if (graph && (!c.graph_exec || c.graph_dt != dt)) {
-        if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
-        c.graph_exec = nullptr;
+        drop_graph(c);
         prepare_assemble(c);
         const bool prof = c.prof;
         c.prof = false;
@@ -1703,6 +1707,7 @@ int bem_get_stats(bem_ctx* c, bem_stats* s) {
 int bem_set_wait_limit(bem_ctx* c, int64_t cycles) {
     CTX_GUARD(c);
     if (cycles <= 0) return c->fail(BEM_ERR_ARG, "bem_set_wait_limit: cycles must be positive");
+    if (c->wait_limit != (long long)cycles) drop_graph(*c);
     c->wait_limit = (long long)cycles;
     return BEM_OK;
 }
