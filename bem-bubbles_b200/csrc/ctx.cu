@@ -847,6 +847,7 @@ int bem_set_params(bem_ctx* c, const bem_params* p) {
     if (!p) return c->fail(BEM_ERR_ARG, "null params");
     const bool to_mixed = p->solver == BEM_SOLVER_MIXED && c->prm.solver != BEM_SOLVER_MIXED;
     if (p->mirror != c->prm.mirror) c->xinv_valid = false;
+    if (memcmp(p, &c->prm, sizeof(*p)) != 0) drop_graph(*c);
     c->prm = *p;
     pred_reset(*c, c->stream);
     if (to_mixed) return ensure_mixed_buffers(*c);

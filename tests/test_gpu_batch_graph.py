@@ -34,3 +34,17 @@ def test_the_wait_limit_reaches_a_captured_step():
     assert np.max(np.abs(a.get_phi() - b.get_phi())) <= 1e-10
     a.close()
     b.close()
+
+
+def test_parameters_reach_a_captured_step():
+    a, b = batch(), batch()
+    a.evolve_graph(2e-3, 1)
+    b.evolve_rk4_steps(2e-3, 1)
+    for bb in (a, b):
+        bb._update(p_inf=2.0, gamma=1.1)
+    a.evolve_graph(2e-3, 2)
+    b.evolve_rk4_steps(2e-3, 2)
+    assert np.array_equal(a.get_vertices(), b.get_vertices())
+    assert np.array_equal(a.get_phi(), b.get_phi())
+    a.close()
+    b.close()
