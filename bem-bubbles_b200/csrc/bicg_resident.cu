@@ -1,7 +1,7 @@
 // BiCGSTAB with the vectors resident on the SMs (the reference's default solver, Simulation.cpp:49-53:
 // Jacobi preconditioner, zero start, tolerance DBL_EPSILON on the recursive residual, at most 2N
 // iterations, shadow-residual restart): the whole solve in one cooperative launch, for N <= 6144.  Up to
-// N = 2048 (33.6 MB) the matrix too stays in the register files and shared memories of the GPU; above, it is
+// N = 2028 (32.9 MB) the matrix too stays in the register files and shared memories of the GPU; above, it is
 // streamed from L2 and HBM.
 //
 // What bounds it, matrix resident: a product reads nothing from outside the SM and takes well under a
@@ -322,10 +322,23 @@ int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaS
     a.ex = reinterpret_cast<ulonglong2*>(c.rbicg);
     a.sc = c.sc;
     a.wait_limit = c.wait_limit;
-    const bool stream = n > RB_RES_N;
     const int np = (n + 1) & ~1, K = (n + RB_T - 1) / RB_T;
     int grid = 0;
-    size_t smem = 0;
+    size_t smem = RB_SMEM + 1;
+    // the matrix on the SMs where a CTA's rows fit: on 148 of them 225.9 KB at N = 2028, 226.1 KB at 2029 (226 at
+    // most); else streamed
+    if (n <= RB_RES_N) {
+        a.rows = std::max(std::min(n, 16), (n + sms - 1) / sms);
+        grid = (n + a.rows - 1) / a.rows;
+        const int cstep = RB_T / a.rows;
+        const int M = K == 1 ? (n <= 8 * cstep ? 8 : 16) : K == 2 ? 28 : K == 3 ? 24 : 20;
+        a.nv = std::max(np, M * cstep);
+        a.nv += a.nv & 1;
+        a.npart = a.rows * (cstep + 1);
+        smem = sizeof(double) *
+               (a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS + (size_t)std::max(0, n - M * cstep) * a.rows);
+    }
+    const bool stream = smem > RB_SMEM;
     if (stream) {
         a.rows = ((n + sms - 1) / sms + 1) & ~1;  // even: a copy takes two rows
         grid = (n + a.rows - 1) / a.rows;
@@ -343,17 +356,6 @@ int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaS
                                           cudaMemcpyDeviceToDevice, s));
             A = c.LU;
         }
-    } else {
-        a.rows = std::max(std::min(n, 16), (n + sms - 1) / sms);
-        grid = (n + a.rows - 1) / a.rows;
-        const int cstep = RB_T / a.rows;
-        const int M = K == 1 ? (n <= 8 * cstep ? 8 : 16) : K == 2 ? 28 : K == 3 ? 24 : 20;
-        a.nv = std::max(np, M * cstep);
-        a.nv += a.nv & 1;
-        a.npart = a.rows * (cstep + 1);
-        smem = sizeof(double) *
-               (a.nv + 2 * (size_t)np + a.npart + 6 * RB_WARPS + (size_t)std::max(0, n - M * cstep) * a.rows);
-        if (smem > RB_SMEM) return BEM_ERR_STATE;
     }
     a.A = A;
     a.seq = ++c.rbicg_solves << 32;
