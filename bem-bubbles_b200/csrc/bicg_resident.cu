@@ -39,6 +39,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "ctx.h"
 #include "resident.cuh"
@@ -378,6 +379,9 @@ int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaS
         c.stats.wait_expired++;
         return c.fail(BEM_ERR_CUDA, "BiCGSTAB: an exchange wait expired");
     }
+    // (alpha / w) / rho, kept for the next beta, leaves the FP64 range where rho falls below 1e-308 (a b of norm 1e-148
+    // or less); beta = (rho / rho_old) (alpha / w), as the other forms have it, does not
+    if (!std::isfinite(c.h_sc->rr)) return BEM_ERR_STATE;
     c.stats.last_iters = c.h_sc->iters;
     c.stats.last_rel_residual = c.h_sc->rhs_sq > 0 ? sqrt(c.h_sc->rr / c.h_sc->rhs_sq) : 0.0;
     c.stats.total_iters += c.stats.last_iters;

@@ -198,7 +198,7 @@ size_t pbicg_words(int64_t n);  // doubles of the persistent BiCGSTAB's dot and 
 // per thread of 512), and of the one whose matrix may too (four; on 148 SMs it fits up to N = 2028).
 constexpr int RB_MAX_N = 12 * 512, RB_RES_N = 4 * 512;
 constexpr double RB_KEEP = 64e6;  // bytes of a streamed matrix kept in L2
-// BEM_OK with the solution in x; BEM_ERR_STATE: not for this size, nothing done; BEM_ERR_CUDA: the
+// BEM_OK with the solution in x; BEM_ERR_STATE: not for this size or these values, the persistent form's; BEM_ERR_CUDA: the
 // launch failed or an exchange wait expired.
 int bicgstab_resident(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s);
 size_t rbicg_words(int64_t n);  // doubles of its exchange slots
