@@ -564,10 +564,10 @@ static int solve_transposed_resident(Ctx& c, const double* G, const double* rhs,
     AdjWork& w = c.adj;
     constexpr int K = 6;
     double h[K + 4];
-    bool first = true;
+    bool renewed = true;
     for (int round = 0; round < 6; ++round) {
         unsigned long long number = 0;
-        if (refine_resident_transposed(c, G, rhs, mu, first, w.xt, K, tol, w.red, &number, s) != BEM_OK) {
+        if (refine_resident_transposed(c, G, rhs, mu, renewed, round == 0, w.xt, K, tol, w.red, &number, s) != BEM_OK) {
             c.rfres_ok = false;
             return BEM_OK;
         }
@@ -578,13 +578,13 @@ static int solve_transposed_resident(Ctx& c, const double* G, const double* rhs,
             c.rfres_ok = false;
             return BEM_OK;
         }
-        first = false;
+        renewed = false;
         *done = h[0] == 0.0 || h[3 + (int)h[1]] <= tol;
         if (*done) return BEM_OK;
         if (round == 1 || round == 3) {  // slow: refresh the approximate inverse against this G
             int rc = mixed_refresh(c, G, s, false);
             if (rc) return rc;
-            first = true;
+            renewed = true;  // mu goes on from where it is
         }
     }
     return c.fail(BEM_ERR_NOT_CONVERGED, "adjoint: transposed solve did not reach the tolerance");

@@ -207,8 +207,8 @@ size_t rbicg_words(int64_t n);  // doubles of its exchange slots
 bool refine_resident_fits(const Ctx& c);
 int refine_resident(Ctx& c, const double* A, const double* b, double* x, const double* r, bool r_ready, int kmax,
                     double tol, double slow, double* out, unsigned long long* number, cudaStream_t s);
-int refine_resident_transposed(Ctx& c, const double* G, const double* b, double* y, bool first, float* xt, int kmax,
-                               double tol, double* out, unsigned long long* number, cudaStream_t s);
+int refine_resident_transposed(Ctx& c, const double* G, const double* b, double* y, bool renewed, bool first, float* xt,
+                               int kmax, double tol, double* out, unsigned long long* number, cudaStream_t s);
 int refine_resident_inverse(Ctx& c, cudaStream_t s);  // after every change of c.Xinv
 size_t refine_resident_words(int64_t n);              // floats of c.Xpad
 // the same for a batch, all blocks in one launch

@@ -446,9 +446,9 @@ __global__ void __launch_bounds__(256)
 }
 
 // The same round for G^T y = b through the transpose of the approximate inverse; xt: n columns of
-// (n + 3) & ~3 floats.  first: the transposes are made and y starts from zero.
-int refine_resident_transposed(Ctx& c, const double* G, const double* b, double* y, bool first, float* xt, int kmax,
-                               double tol, double* out, unsigned long long* number, cudaStream_t s) {
+// (n + 3) & ~3 floats.  renewed: G or the inverse changed, the transposes are made; first: y starts from zero.
+int refine_resident_transposed(Ctx& c, const double* G, const double* b, double* y, bool renewed, bool first, float* xt,
+                               int kmax, double tol, double* out, unsigned long long* number, cudaStream_t s) {
     const int n = (int)c.topo.N, nt = (n + 31) / 32;
     RSys a{};
     a.n = n;
@@ -459,10 +459,8 @@ int refine_resident_transposed(Ctx& c, const double* G, const double* b, double*
     a.b = b;
     a.r = first ? b : nullptr;
     a.x = y;
-    if (first) {
-        KLAUNCH(), k_transpose_gx<<<dim3(nt, nt, 2), 256, 0, s>>>(n, G, c.Xinv, c.LU, a.ldg, xt, a.ldx);
-        BEM_CUDA(c, cudaMemsetAsync(y, 0, sizeof(double) * n, s));
-    }
+    if (renewed) KLAUNCH(), k_transpose_gx<<<dim3(nt, nt, 2), 256, 0, s>>>(n, G, c.Xinv, c.LU, a.ldg, xt, a.ldx);
+    if (first) BEM_CUDA(c, cudaMemsetAsync(y, 0, sizeof(double) * n, s));
     // the separate launches always run six steps: two orders below the tolerance, or one step past it
     const RRule q = rr_rule(c, n, kmax, tol, tol >= 1e-13 ? 0.01 : 1.0, INFINITY);
     return rr_round(c, a, q, out, number, s);
