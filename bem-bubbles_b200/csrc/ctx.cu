@@ -644,7 +644,8 @@ static int alloc_mixed(Ctx& c) {
         (rc = dalloc(c, &planes, 4 * np)) || (rc = dalloc(c, &c.tc_err, 1)) ||
         (rc = dalloc(c, &c.V, n * (size_t)(c.gmres_m + 1))) || (rc = dalloc(c, &c.Z, n * (size_t)c.gmres_m)))
         return rc;
-    if (refine_resident_words(c.topo.N) && (rc = dalloc(c, &c.Xpad, refine_resident_words(c.topo.N)))) return rc;
+    if (refine_resident_words(c.topo.N) && dalloc(c, &c.Xpad, refine_resident_words(c.topo.N)))
+        cudaGetLastError();  // no memory for the padded copy: the separate launches
     c.tcp = planes;
     BEM_CUDA(c, cudaMemset(c.tc_err, 0, sizeof(int)));
     return BEM_OK;

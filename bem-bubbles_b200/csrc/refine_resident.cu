@@ -528,13 +528,12 @@ int refine_batch_setup(Ctx& c) {
     if ((rc = upload_vec(c, &c.blist, list)) || (rc = upload_vec(c, &c.boff, off)) ||
         (rc = upload_vec(c, &c.bxoff, xoff)) ||
         (rc = dalloc(c, &c.bslots, 4 * (size_t)c.h_blk.back().vbase + 4 * (size_t)c.h_blk.back().n)) ||
-        (rc = dalloc(c, &c.bnumber, 1)))
-        return rc;
-    c.h_bxoff = xoff;
-    if (dalloc(c, &c.Xbpad, (size_t)xtot)) {  // no memory for the copies: the separate launches
-        cudaGetLastError();
+        (rc = dalloc(c, &c.bnumber, 1)) || (rc = dalloc(c, &c.Xbpad, (size_t)xtot))) {
+        if (rc != BEM_ERR_NOMEM) return rc;
+        cudaGetLastError();  // no memory for the copies: the separate launches
         return BEM_OK;
     }
+    c.h_bxoff = xoff;
     BEM_CUDA(c, cudaMemset(c.bslots, 0, sizeof(double) * 4 * (size_t)(c.h_blk.back().vbase + c.h_blk.back().n)));
     BEM_CUDA(c, cudaMemset(c.bnumber, 0, sizeof(unsigned long long)));
     c.bteam = team;
