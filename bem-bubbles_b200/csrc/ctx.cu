@@ -640,12 +640,19 @@ static int alloc_mixed(Ctx& c) {
     const size_t n = (size_t)c.topo.N, nn = n * n, np = (size_t)tc_pad((int)n) * tc_pad((int)n);
     uint16_t* planes = nullptr;
     int rc;
-    if ((rc = dalloc(c, &c.Xinv, nn)) || (rc = dalloc(c, &c.Tw, nn)) || (rc = dalloc(c, &c.G32, nn)) ||
-        (rc = dalloc(c, &planes, 4 * np)) || (rc = dalloc(c, &c.tc_err, 1)) ||
-        (rc = dalloc(c, &c.V, n * (size_t)(c.gmres_m + 1))) || (rc = dalloc(c, &c.Z, n * (size_t)c.gmres_m)))
+    if ((rc = dalloc(c, &c.Tw, nn)) || (rc = dalloc(c, &c.G32, nn)) || (rc = dalloc(c, &planes, 4 * np)) ||
+        (rc = dalloc(c, &c.tc_err, 1)) || (rc = dalloc(c, &c.V, n * (size_t)(c.gmres_m + 1))) ||
+        (rc = dalloc(c, &c.Z, n * (size_t)c.gmres_m)))
         return rc;
-    if (refine_resident_words(c.topo.N) && dalloc(c, &c.Xpad, refine_resident_words(c.topo.N)))
-        cudaGetLastError();  // no memory for the padded copy: the separate launches
+    // the inverse and behind it its padded copy (resident refinement) in one allocation: a small context's set-up
+    // is its allocations.  The last one: without room for both the inverse alone, and separate launches.
+    const size_t words = refine_resident_words(c.topo.N), pad = (nn + 63) & ~(size_t)63;  // 256 bytes
+    if (words && dalloc(c, &c.Xinv, pad + words) == BEM_OK) {
+        c.Xpad = c.Xinv + pad;
+    } else {
+        cudaGetLastError();
+        if ((rc = dalloc(c, &c.Xinv, nn))) return rc;
+    }
     c.tcp = planes;
     BEM_CUDA(c, cudaMemset(c.tc_err, 0, sizeof(int)));
     return BEM_OK;
@@ -716,7 +723,9 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
                        &c.kp3, &c.kp4, &c.r, &c.r0, &c.pv, &c.vv, &c.yv, &c.zv, &c.sv, &c.tv, &c.invd, &c.potz};
     for (auto p : vecs)
         if ((rc = dalloc(c, p, n))) return rc;
-    if ((rc = dalloc(c, &c.G, nn)) || (rc = dalloc(c, &c.H, nn)) || (!c.batch && (rc = dalloc(c, &c.LU, nn + n))) ||
+    // the step path writes no H: its storage holds the halo columns (more than H in small systems of small patches)
+    const size_t nh = std::max(nn, (size_t)(t.npatch > 0 ? h.halo_elems : 0));
+    if ((rc = dalloc(c, &c.G, nn)) || (rc = dalloc(c, &c.H, nh)) || (!c.batch && (rc = dalloc(c, &c.LU, nn + n))) ||
         (rc = dalloc(c, &c.rec, m * REC)) || (rc = dalloc(c, &c.tn, 3 * m)) || (rc = dalloc(c, &c.tg, 3 * m)) ||
         (rc = dalloc(c, &c.tk, m)) || (rc = dalloc(c, &c.rowHp, nrow_part)) ||
         (rc = dalloc(c, &c.bp, nrow_part)) || (!c.batch && (rc = dalloc(c, &c.gp, nrow_part))) || (rc = dalloc(c, &c.vol, (size_t)h.nparts + 1)) ||
@@ -730,14 +739,10 @@ static int alloc_mesh(Ctx& c, int64_t N, int64_t M, const HostTopo& h) {
         return rc;
     if (c.psih_t) BEM_CUDA(c, cudaMemset(c.psih_t, 0, sizeof(double) * (PRED_CNT + 1)));
     if (t.npatch > 0) {
-        // the step path writes no H: its storage holds the halo columns when they fit
         if ((rc = dalloc(c, &c.prec, m * PREC)) || (rc = dalloc(c, &c.asm_err, 4)) || (rc = dalloc(c, &c.rf_bar, RF_WORDS)))
             return rc;
         BEM_CUDA(c, cudaMemset(c.rf_bar, 0, sizeof(int) * RF_WORDS));
-        if ((size_t)h.halo_elems <= nn)
-            c.halo = c.H;
-        else if ((rc = dalloc(c, &c.halo, (size_t)h.halo_elems)))
-            return rc;
+        c.halo = c.H;
         BEM_CUDA(c, cudaMemset(c.asm_err, 0, sizeof(int) * 4));
     }
     if (!c.batch && c.prm.solver == BEM_SOLVER_MIXED) {
