@@ -1003,8 +1003,9 @@ int lu_solve(Ctx& c, const double* A, const double* b, double* x, cudaStream_t s
         if (!done) c.lu_rows_ok = false;  // factor again with the single-CTA panel
     }
     if (!done) {
-        if ((size_t)n * sizeof(double) > 200 * 1024)
-            return c.fail(BEM_ERR_ARG, "LU solver: N too large for the single-CTA panel (N <= 25600)");
+        // One CTA for every panel: 97 ms a solve at N = 4002 (8.2 with the panels spread), 0.37 s at 7842 (0.03),
+        // 1.6 s at 16002 (0.19), about four seconds at the limit.  Past it a solve is refused.
+        if (n > 25600) return c.fail(BEM_ERR_ARG, "LU solver: N too large for the single-CTA panel (N <= 25600)");
         if ((rc = lu_factor(c, A, b, s, false)) || (rc = lu_back_substitute(c, x, s)) || (rc = status())) return rc;
     }
     if (c.h_flag[0] & 2) {  // a wait of the back substitution expired: one launch per row block
