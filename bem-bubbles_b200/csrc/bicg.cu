@@ -4,7 +4,8 @@
 // runs a batch of iterations per launch.
 //
 // One BiCGSTAB iteration is two GEMVs and three vector updates; as separate launches it is about
-// nine kernels.  This form serves N > 6144 (smaller systems: bicg_resident.cu).  Here the phases are
+// nine kernels.  This form serves N > 6144, and below (bicg_resident.cu) more than 24576 iterations and
+// right-hand sides of norm 1e-148 or less.  Here the phases are
 // separated by a grid-wide barrier (sense counter in global memory, bounded wait), the scalars are
 // recomputed redundantly by every CTA from the same per-row-block partial sums (fixed order, so every
 // CTA holds the same bits), and the host polls the done flag once per batch of iterations.

@@ -11,7 +11,8 @@
 // four steps: 38 us (about 105, with the gaps).
 // In a batch a team of CTAs takes one block after another, so that no stage waits for the slowest block between
 // its products: four stages of 24 blocks of 362 to 1442 unknowns 5.16 -> 4.16 ms, of 256 of them 53.1 -> 51.0 ms
-// (the matrices then come from HBM either way: 31 B per clock and SM).
+// (the matrices then come from HBM either way: 31 B per clock and SM; of one stage of 24 blocks 386 of the 514 MB that
+// its products read).
 #include <math.h>
 
 #include <algorithm>
@@ -258,8 +259,9 @@ struct BRArgs {
     int team, nv, npart;
 };
 
-// A batch: teams of CTAs take their blocks one after the other, so that a block's G and X are read from HBM
-// once and from L2 in the steps after the first.
+// A batch: teams of CTAs take their blocks one after the other.  The steps after a block's first find in L2 what is
+// left there of its G and X beside the other teams' blocks: a quarter of the reads with 24 blocks, next to nothing
+// in a large sweep.
 template <int K>
 __global__ void __launch_bounds__(RB_T, 1) k_refine_batch(const BRArgs a, const RRule q) {
     extern __shared__ __align__(16) double smem[];
@@ -555,8 +557,8 @@ int refine_batch_inverse(Ctx& c, int b, cudaStream_t s) {
 int refine_batch(Ctx& c, const double* A, const double* b, double* x, int kmax, double tol, double* err, cudaStream_t s) {
     BRArgs a{c.blk, c.blist, c.boff, c.bxoff, A, c.Xb, c.Xbpad, b, x, reinterpret_cast<ulonglong2*>(c.bslots),
              (long long)c.topo.N, c.bnumber, c.bstat, err, c.bconv, c.bteam, c.bnv, c.bnpart};
+    // Everything marked to stay is no preference, and none helps: a share for G changed nothing
     RRule q{kmax, tol, 1.0, INFINITY, c.wait_limit, 1.0f, 1.0f};
-
     KLAUNCH(), k_next_number<<<1, 1, 0, s>>>(c.bnumber);
     void* args[] = {&a, &q};
     KLAUNCH();

@@ -76,11 +76,11 @@ typedef struct {
  * H.  Both give the same G and b to rounding; for comparison. */
 #define BEM_FLAG_STEP_ASSEMBLE_H 4
 /* bem_params.flags: run each round of BEM_SOLVER_MIXED's refinement steps as one cooperative kernel
- * with grid barriers over the tiles of the separate GEMV launches (the same summation order:
- * bit-identical results, with BEM_FLAG_NO_IR_GATE).  Measured slower than the separate launches on
+ * with grid barriers over the tiles of k_gemv (bit-identical, with BEM_FLAG_NO_IR_GATE, to the separate
+ * launches where those use k_gemv: N below 4700, or odd; larger even systems sum in another order).  Measured slower than the separate launches on
  * B200 (0.36 against 0.27 ms per solve at N = 4002), and those slower than the default for N <= 6144,
  * a cooperative launch whose vectors stay on the SMs and whose convergence test is on the device
- * (0.21 ms).  For comparison. */
+ * (0.18 ms).  For comparison. */
 #define BEM_FLAG_REFINE_PERSISTENT 8
 /* bem_params.flags: how BEM_SOLVER_MIXED builds its approximate inverse from scratch.  By default
  * (neither flag) large systems (N >= BEM_GJ_MIN_N) use blocked Gauss-Jordan elimination with row
@@ -151,7 +151,8 @@ int bem_assemble_rhs(bem_ctx* ctx, const double* verts, const double* pot, doubl
 /* Simulation::solve_system (Simulation.cpp:40-71): x = G^{-1} b with the context's solver. */
 int bem_solve_system(bem_ctx* ctx, const double* G, const double* b, double* x);
 /* LinLinSim::position_t (LinLinSim.cpp:26-83): vertex velocities for positions `verts` (NULL = mesh)
- * and potential `pot`.  psi_l (the solved dphi/dn) may be NULL. */
+ * and potential `pot`.  psi_l (the solved dphi/dn) may be NULL.  On a batch every block is solved;
+ * BEM_ERR_NOT_CONVERGED when one misses the tolerance with a renewed inverse. */
 int bem_position_t(bem_ctx* ctx, const double* verts, const double* pot, double* vel, double* psi_l);
 /* bem_position_t with pot in/out, as the reference's PotVec& argument: with pinned vertices
  * (bem_set_pinned) pot receives the solved potential at the pinned vertices (ColocSimPin.cpp:188). */
@@ -290,13 +291,14 @@ typedef struct {
 int bem_get_stats(bem_ctx* ctx, bem_stats* s);
 
 /* Bound, in SM clock cycles, of every grid-wide barrier or exchange wait of the persistent kernels (the
- * cooperative BiCGSTAB forms, the cooperative refinement rounds of a system and of a batch, the
- * row-distributed LU panel) and of the LU cluster panel's and back substitution's waits.  Default 2e9 (about a second at the B200's clock).  A wait that
- * runs out makes the kernel set its error word and return; the host reads it, counts it in
- * bem_stats.wait_expired and finishes the solve with the multi-kernel form (for the LU: the
- * single-CTA panel), which the context keeps for the rest of its life.  No counterpart in the reference (its solves
- * run on the host); exists so that this failure path can be tested without a GPU fault.
- * cycles <= 0 returns BEM_ERR_ARG. */
+ * cooperative BiCGSTAB forms, the cooperative refinement rounds of a system, its transpose and a batch,
+ * the row-distributed LU panel) and of the LU cluster panel's and back substitution's waits.  Default
+ * 2e9 (about a second at the B200's clock).  A wait that runs out makes the kernel set its error word and
+ * return; the host reads it, counts it in bem_stats.wait_expired and finishes the solve with the
+ * multi-kernel form (for the LU: the single-CTA panel), which the context keeps for the rest of its life
+ * (a batch: of its mesh).  No counterpart in the reference (its solves run on the host); exists so that this failure path can be tested without a GPU fault.
+ * A captured batch step (bem_evolve_rk4_graph) is captured again with a changed limit, as with changed
+ * parameters (bem_set_params).  cycles <= 0 returns BEM_ERR_ARG. */
 int bem_set_wait_limit(bem_ctx* ctx, int64_t cycles);
 
 /* Synchronise the context's stream. */
